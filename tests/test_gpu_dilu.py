@@ -138,9 +138,52 @@ def test_dilu_batch_matches_solo():
         off += g["n_cells"]
 
 
+@pytest.mark.parametrize("n,periodic,two_d", [
+    ((97, 83, 1), (0, 0, 0), True),      # too many rows for one CTA, narrow levels: steps of one part, few mailboxes
+    ((41, 35, 29), (1, 0, 1), False),    # parts cut inside planes; periodic links reach back over many parts
+    ((64, 64, 64), (1, 1, 1), False),    # levels wider than a step
+    ((150, 140, 130), (0, 0, 0), False),  # more rows than the parts' shared memory holds
+])
+def test_pipelined_parts_apply_bitwise(n, periodic, two_d):
+    """Systems too wide for one CTA: factor, forward and backward sweeps over parts that exchange
+    mailboxes equal the natural-order ones bit for bit, also when repeated (stale mailboxes)."""
+    from voluma_b200 import mesh as vm
+    msh = vb.box_mesh_device(n, hi=(1.0, 1.0, 1.0), periodic=periodic, two_d=two_d)
+    diag, upper = vm.poisson_matrix(msh)
+    rng = np.random.default_rng(7)
+    lower = upper * (0.8 + 0.4 * rng.random(msh["n_internal_faces"]))
+    m = vb.Mesh.from_arrays(msh)
+    for _ in range(2):
+        r = rng.standard_normal(msh["n_cells"])
+        w = vb.precond_apply(m, diag, upper, lower, r, "DILU")
+        assert np.array_equal(w, ro.precond_apply(msh, diag, upper, lower, r, "DILU"))
+
+
+def test_pipelined_parts_of_a_batch_match_solo():
+    """Two wide systems of a batch: their parts share one launch, each result its own."""
+    from voluma_b200 import mesh as vm
+    msh = [vm.box_mesh(n, hi=(1.0, 1.0, 1.0)) for n in ((44, 40, 36), (33, 39, 35))]
+    mats = [vm.poisson_matrix(q) for q in msh]
+    rng = np.random.default_rng(11)
+    lows = [u * (0.8 + 0.4 * rng.random(u.size)) for _, u in mats]
+    b = [rng.standard_normal(q["n_cells"]) for q in msh]
+    ctrl = vb.SolverControls("PBiCGStab", "DILU", 0.0, 1e-6, 50)
+    batch = vb.Mesh.batch(msh)
+    x = np.zeros(batch.n_cells)
+    perfs = vb.solve_ldu(batch, np.concatenate([d for d, _ in mats]), np.concatenate([u for _, u in mats]),
+                         np.concatenate(lows), np.concatenate(b), x, ctrl)
+    off = 0
+    for q, (d, u), lo, rhs, p in zip(msh, mats, lows, b, perfs):
+        xs = np.zeros(q["n_cells"])
+        ps = vb.solve_ldu(vb.Mesh.from_arrays(q), d, u, lo, rhs, xs, ctrl)
+        assert np.array_equal(x[off:off + q["n_cells"]], xs) and p.iterations == ps.iterations
+        off += q["n_cells"]
+
+
 def test_wide_system_uses_a_cooperative_group():
     """48^3 box: levels up to ~1700 rows wide, so one system is swept by a co-resident group of CTAs
-    with the bounded global barrier; the result is still the natural-order one, bit for bit."""
+    with the bounded global barrier (Gauss-Seidel) or by pipelined parts (DILU); the result is still
+    the natural-order one, bit for bit."""
     from voluma_b200 import mesh as vm
     msh = vm.box_mesh((48, 48, 48), hi=(1.0, 1.0, 1.0), periodic=(0, 0, 0))
     diag, upper = vm.poisson_matrix(msh)

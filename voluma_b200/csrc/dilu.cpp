@@ -121,4 +121,103 @@ DiluPlan buildDiluPlan(const std::vector<SysTopo>& systems, const BatchPlan& P) 
     return D;
 }
 
+DiluParts buildDiluParts(const DiluPlan& D, const BatchPlan& P, const std::vector<int>& nParts, int maxWidth) {
+    DiluParts R;
+    const int nrows = int(P.perm0.size());
+    std::vector<int32_t> partOf(size_t(nrows), -1), slotOf(size_t(nrows), -1);
+    // slots: per part and level the rows of that level, in steps of at most maxWidth
+    for (const DiluSys& ds : D.sys) {
+        const int64_t n = P.sysCells[ds.sys], cb = P.userCellBase[P.order[ds.sys]];
+        const int np = std::max(1, std::min<int>(nParts[ds.sys], int(std::max<int64_t>(n, 1))));
+        const int part0 = int(R.parts.size());
+        std::vector<std::vector<int32_t>> rows(static_cast<size_t>(np));  // level by level
+        std::vector<std::vector<int32_t>> ends(static_cast<size_t>(np));  // end of each non-empty level's rows
+        for (int t = 0; t < ds.nLev; ++t) {
+            for (int k = D.levPtr[ds.levBegin + t]; k < D.levPtr[ds.levBegin + t + 1]; ++k) {
+                const int r = D.levRows[k];
+                if (P.perm0[r] < 0) continue;  // padding: never written, no neighbours
+                const int q = int((P.perm0[r] - cb) * np / n);
+                partOf[r] = part0 + q;
+                rows[q].push_back(r);
+            }
+            for (int q = 0; q < np; ++q)
+                if (int(rows[q].size()) > (ends[q].empty() ? 0 : ends[q].back())) ends[q].push_back(int(rows[q].size()));
+        }
+        for (int q = 0; q < np; ++q) {
+            DiluPart part{ds.sys, int(R.steps.size()), 0, int(R.slotRow.size()), int(rows[q].size())};
+            int a = 0;
+            for (int e : ends[q])
+                while (a < e) {
+                    const int w = std::min(maxWidth, e - a);
+                    DiluStep st = {};
+                    st.s0 = part.slot0 + a;
+                    st.width = w;
+                    R.steps.push_back(st);
+                    R.maxWidth = std::max(R.maxWidth, w);
+                    a += w;
+                }
+            part.nSteps = int(R.steps.size()) - part.stepBegin;
+            for (int r : rows[q]) {
+                slotOf[r] = int(R.slotRow.size());
+                R.slotRow.push_back(r);
+            }
+            R.maxSlots = std::max(R.maxSlots, part.nSlots);
+            R.parts.push_back(part);
+        }
+    }
+    // mailboxes: one per row read by another part, per direction
+    R.loMail.assign(R.slotRow.size(), -1);
+    R.upMail.assign(R.slotRow.size(), -1);
+    for (int r : R.slotRow) {
+        for (int k = D.loPtr[r]; k < D.loPtr[r + 1]; ++k)
+            if (partOf[D.loCol[k]] != partOf[r] && R.loMail[slotOf[D.loCol[k]]] < 0)
+                R.loMail[slotOf[D.loCol[k]]] = R.nLoMail++;
+        for (int k = D.upPtr[r]; k < D.upPtr[r + 1]; ++k)
+            if (partOf[D.upCol[k]] != partOf[r] && R.upMail[slotOf[D.upCol[k]]] < 0)
+                R.upMail[slotOf[D.upCol[k]]] = R.nUpMail++;
+    }
+    // entries, column-major per step
+    auto fill = [&](const DiluPart& part, const DiluStep& st, const std::vector<int32_t>& ptr,
+                    const std::vector<int32_t>& col, const std::vector<int32_t>& face,
+                    const std::vector<int32_t>& mail, std::vector<int32_t>& outCol, std::vector<int32_t>& outFace,
+                    std::vector<int32_t>& remote, int& e0, int& m, int& r0, int& nr) {
+        e0 = int(outCol.size());
+        r0 = int(remote.size());
+        m = 0;
+        for (int q = 0; q < st.width; ++q) {
+            const int r = R.slotRow[st.s0 + q];
+            m = std::max(m, int(ptr[r + 1] - ptr[r]));
+        }
+        for (int j = 0; j < m; ++j)
+            for (int q = 0; q < st.width; ++q) {
+                const int r = R.slotRow[st.s0 + q];
+                const int k = ptr[r] + j;
+                if (k >= ptr[r + 1]) {
+                    outCol.push_back(-1);
+                    outFace.push_back(0);
+                    continue;
+                }
+                const int c = col[k];
+                if (partOf[c] == partOf[r]) {
+                    outCol.push_back(slotOf[c] - part.slot0);
+                } else {
+                    outCol.push_back(-2 - (int(remote.size()) - r0));
+                    remote.push_back(mail[slotOf[c]]);
+                }
+                outFace.push_back(face[k]);
+            }
+        nr = int(remote.size()) - r0;
+        R.maxRemote = std::max(R.maxRemote, nr);
+    };
+    for (const DiluPart& part : R.parts)
+        for (int t = part.stepBegin; t < part.stepBegin + part.nSteps; ++t) {
+            DiluStep& st = R.steps[t];
+            fill(part, st, D.loPtr, D.loCol, D.loFace, R.loMail, R.loCol, R.loFace, R.loRemote, st.lo, st.mlo, st.rlo,
+                 st.nrlo);
+            fill(part, st, D.upPtr, D.upCol, D.upFace, R.upMail, R.upCol, R.upFace, R.upRemote, st.up, st.mup, st.rup,
+                 st.nrup);
+        }
+    return R;
+}
+
 }  // namespace vlm

@@ -1,12 +1,14 @@
 // Level-scheduled kernels: DIC/DILU factorisation and application (LinearSolver.cpp:56-112), and
 // the Gauss-Seidel / symmetric Gauss-Seidel / Jacobi solvers (LinearSolver.cpp:238-278).
 //
-// One group of G CTAs works on one system and walks its levels (dilu.h) in order; rows of one
-// level are independent, so they are spread over the group's threads, and the group synchronises
-// between levels.  With G == 1 that is __syncthreads(); with G > 1 (one large system, launched
-// cooperatively so the group is co-resident) it is a counter barrier in global memory whose wait
-// gives up after a bounded number of polls, sets VLM_ERR_TIMEOUT in *err and lets the kernel run
-// to its end.  Values written by other CTAs of the group are read through L2 (ld.global.cg).
+// DIC/DILU sweeps: one CTA per system where its vector fits in shared memory (below), else the
+// pipelined parts of dilupart.cuh.  Gauss-Seidel: one group of G CTAs works on one system and walks
+// its levels (dilu.h) in order; rows of one level are independent, so they are spread over the group's
+// threads, and the group synchronises between levels.  With G == 1 that is __syncthreads(); with G > 1
+// (one large system, launched cooperatively so the group is co-resident) it is a counter barrier in
+// global memory whose wait gives up after a bounded number of polls, sets VLM_ERR_TIMEOUT in *err and
+// lets the kernel run to its end.  Values written by other CTAs of the group are read through L2
+// (ld.global.cg).
 #pragma once
 
 #include "krylov.cuh"
@@ -69,89 +71,6 @@ __global__ void k_group_barrier_check(DiluBar* bar, int G, int* err, long long s
     for (int idx = levPtr[(d).levBegin + (t)] + tid; idx < levPtr[(d).levBegin + (t) + 1]; \
          idx += nthr)
 
-// Per-solve coefficients in schedule order: A_ul and A_lu of every lower entry, A_lu of every
-// upper entry (LinearSolver.cpp:70-72, 99, 104).
-__global__ void k_dilu_values(int n, const int32_t* __restrict__ loFace, const int32_t* __restrict__ upFace,
-                              const double* __restrict__ upper, const double* __restrict__ lower,
-                              double* __restrict__ loAul, double* __restrict__ loAlu, double* __restrict__ upAlu) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const int32_t a = loFace[k], b = upFace[k];
-    const int fa = a & 0x7fffffff, fb = b & 0x7fffffff;
-    const bool la = a < 0, lb = b < 0;  // ownerIsL
-    loAul[k] = la ? lower[fa] : upper[fa];
-    loAlu[k] = la ? upper[fa] : lower[fa];
-    upAlu[k] = lb ? upper[fb] : lower[fb];
-}
-
-// rD[u] = D[u] - sum_l A_lu A_ul / rD[l] in level order, then rD = 1 / rD (LinearSolver.cpp:66-77)
-__global__ void __launch_bounds__(kDiluThreads) k_dilu_factor(const DiluSys* __restrict__ ds, int G,
-                                                              const int32_t* __restrict__ levPtr,
-                                                              const int32_t* __restrict__ levRows,
-                                                              const int32_t* __restrict__ loPtr,
-                                                              const int32_t* __restrict__ loCol,
-                                                              const double* __restrict__ loAlu,
-                                                              const double* __restrict__ loAul,
-                                                              const double* __restrict__ diag, double* rD,
-                                                              DiluBar* bars, int* err) {
-    const DiluSys d = ds[blockIdx.x / G];
-    const int tid = int(blockIdx.x % G) * blockDim.x + threadIdx.x, nthr = G * blockDim.x;
-    DiluBar* bar = bars + blockIdx.x / G;
-    for (int t = 0; t < d.nLev; ++t) {
-        VLM_LEVEL_ROWS(d, t, idx) {
-            const int c = levRows[idx];
-            double v = diag[c];
-            for (int k = loPtr[c]; k < loPtr[c + 1]; ++k) v -= loAlu[k] * loAul[k] / __ldcg(rD + loCol[k]);
-            rD[c] = v;
-        }
-        group_sync(bar, G, err);
-    }
-    for (int t = 0; t < d.nLev; ++t) VLM_LEVEL_ROWS(d, t, idx) {
-            const int c = levRows[idx];
-            rD[c] = 1.0 / __ldcg(rD + c);
-        }
-}
-
-// w = M^-1 r: w = rD r; forward w[u] -= rD[u] A_ul w[l]; backward w[l] -= rD[l] A_lu w[u]
-// (LinearSolver.cpp:87-106)
-__global__ void __launch_bounds__(kDiluThreads) k_dilu_apply(const DiluSys* __restrict__ ds, int G,
-                                                             const int32_t* __restrict__ levPtr,
-                                                             const int32_t* __restrict__ levRows,
-                                                             const int32_t* __restrict__ loPtr,
-                                                             const int32_t* __restrict__ loCol,
-                                                             const double* __restrict__ loAul,
-                                                             const int32_t* __restrict__ upPtr,
-                                                             const int32_t* __restrict__ upCol,
-                                                             const double* __restrict__ upAlu,
-                                                             const double* __restrict__ rD, const double* r, double* w,
-                                                             DiluBar* bars, int* err, const SysState* st, int flag) {
-    pdl_entry();
-    const DiluSys d = ds[blockIdx.x / G];
-    if (st != nullptr && sys_idle(st[d.sys], flag)) return;  // uniform over the group
-    const int tid = int(blockIdx.x % G) * blockDim.x + threadIdx.x, nthr = G * blockDim.x;
-    DiluBar* bar = bars + blockIdx.x / G;
-    for (int t = 0; t < d.nLev; ++t) {
-        VLM_LEVEL_ROWS(d, t, idx) {
-            const int c = levRows[idx];
-            const double rd = rD[c];
-            double wc = rd * r[c];
-            for (int k = loPtr[c]; k < loPtr[c + 1]; ++k) wc -= rd * loAul[k] * __ldcg(w + loCol[k]);
-            w[c] = wc;
-        }
-        group_sync(bar, G, err);
-    }
-    for (int t = d.nLev - 1; t >= 0; --t) {
-        VLM_LEVEL_ROWS(d, t, idx) {
-            const int c = levRows[idx];
-            const double rd = rD[c];
-            double wc = __ldcg(w + c);
-            for (int k = upPtr[c]; k < upPtr[c + 1]; ++k) wc -= rd * upAlu[k] * __ldcg(w + upCol[k]);
-            w[c] = wc;
-        }
-        if (t > 0) group_sync(bar, G, err);
-    }
-}
-
 // ---------------------------------------------------------------- shared-memory (streamed) variants
 // One CTA per system whose level-0 vector fits in shared memory and whose levels are at most one
 // row per thread.  The swept vector lives in shared memory.  The schedule is streamed (dilu.h,
@@ -161,7 +80,7 @@ __global__ void __launch_bounds__(kDiluThreads) k_dilu_apply(const DiluSys* __re
 //
 // The factor's A_lu * A_ul is formed once per factorisation (the product the reference's
 // rD[u] -= A_lu A_ul / rD[l] forms first); every other operation is the reference's, in its order,
-// so the results are those of k_dilu_factor / k_dilu_apply bit for bit.
+// so the results are the reference's bit for bit.
 constexpr int kDiluRing = 8;
 
 __device__ __forceinline__ void cp_async4(void* dst, const void* src) {
@@ -269,16 +188,17 @@ __device__ __forceinline__ char* dilu_stream_setup(char* smem, const DiluSys& d,
 }
 
 // Per-solve coefficients of the streamed schedule: prod = A_lu A_ul and coefLo = A_ul per lower
-// entry, coefUp = A_lu per upper entry.
+// entry, coefUp = A_lu per upper entry (column -1: padding).
 __global__ void k_dilu_stream_values(int nLo, int nUp, const int32_t* __restrict__ loCol,
                                      const int32_t* __restrict__ loFace, const int32_t* __restrict__ upCol,
                                      const int32_t* __restrict__ upFace, const double* __restrict__ upper,
                                      const double* __restrict__ lower, double* __restrict__ prod,
                                      double* __restrict__ coefLo, double* __restrict__ coefUp) {
+    pdl_entry();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k < nLo) {
         double p = 0.0, c = 0.0;
-        if (loCol[k] >= 0) {
+        if (loCol[k] != -1) {
             const int32_t a = loFace[k];
             const int fa = a & 0x7fffffff;
             const double aul = a < 0 ? lower[fa] : upper[fa];
@@ -291,7 +211,7 @@ __global__ void k_dilu_stream_values(int nLo, int nUp, const int32_t* __restrict
     } else if (k - nLo < nUp) {
         const int q = k - nLo;
         double c = 0.0;
-        if (upCol[q] >= 0) {
+        if (upCol[q] != -1) {
             const int32_t b = upFace[q];
             const int fb = b & 0x7fffffff;
             c = b < 0 ? upper[fb] : lower[fb];

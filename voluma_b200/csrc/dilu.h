@@ -57,4 +57,34 @@ struct DiluPlan {
 // systems: input order; P: the batch plan (solver order, perm0).
 DiluPlan buildDiluPlan(const std::vector<SysTopo>& systems, const BatchPlan& P);
 
+// Pipelined schedule of systems too wide for one CTA: the rows of a system are cut into parts of
+// consecutive natural rows, one CTA each.  A lower neighbour precedes its row in natural order, so a
+// part's forward sweep reads only its own rows and rows of earlier parts (its backward sweep, of
+// later parts): each part walks its own rows level by level and takes the values of other parts from
+// per-value mailboxes, so no two CTAs ever meet at a barrier.  Slots: every real row of a part, step by
+// step; a step is at most maxWidth rows of one level.
+struct DiluPart {
+    int sys, stepBegin, nSteps, slot0, nSlots;
+};
+
+// Slots [s0, s0 + width); entry j of slot s0 + q at lo + j * width + q (up likewise): a slot of the part
+// relative to its slot0, -1 padding, or -2 - k: the step's remote entry k (mailbox loRemote[rlo + k]).
+struct DiluStep {
+    int s0, width, lo, mlo, up, mup, rlo, nrlo, rup, nrup;
+};
+
+struct DiluParts {
+    std::vector<DiluPart> parts;  // forward order; the backward sweep takes them in reverse
+    std::vector<DiluStep> steps;
+    std::vector<int32_t> slotRow;                        // slot -> solver row
+    std::vector<int32_t> loCol, loFace, upCol, upFace;   // entries (faces as DiluPlan's)
+    std::vector<int32_t> loRemote, upRemote;             // mailbox of each remote entry
+    std::vector<int32_t> loMail, upMail;                 // per slot: the mailbox its value goes to, -1: none
+    int nLoMail = 0, nUpMail = 0;
+    int maxSlots = 0, maxWidth = 0, maxRemote = 0;
+};
+
+// nParts[b]: parts of the system at batch position b (at least 1).
+DiluParts buildDiluParts(const DiluPlan& D, const BatchPlan& P, const std::vector<int>& nParts, int maxWidth);
+
 }  // namespace vlm

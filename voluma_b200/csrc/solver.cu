@@ -15,6 +15,7 @@
 #include "boxkernels.cuh"
 #include "boxstream.cuh"
 #include "dilu.cuh"
+#include "dilupart.cuh"
 #include "krylov.cuh"
 #include "aggl.h"
 #include "solver.h"
@@ -24,12 +25,12 @@ namespace vlm {
 
 // Device copy of the level schedule (dilu.h) and the per-solve DIC/DILU arrays.
 struct DiluDev {
-    DBuf<int32_t> loPtr, loCol, loFace, upPtr, upCol, upFace, levPtr, levRows;
+    DBuf<int32_t> levPtr, levRows;
     DBuf<DiluSys> sys;
-    DBuf<double> loAul, loAlu, upAlu, rD;
     DBuf<DiluBar> bars;
     DBuf<int> err;
-    int G = 1, groups = 0, nFaces = 0;
+    int G = 1, groups = 0;  // Gauss-Seidel sweeps: CTAs per system
+    bool groupSweeps = false;  // a cooperative (G > 1) sweep has been recorded
     // streamed shared-memory sweeps (dilu.h DiluLevel): used when smem > 0
     DBuf<DiluLevel> lev;
     DBuf<int32_t> slotRow, sLoCol, sLoFace, sUpCol, sUpFace;
@@ -37,6 +38,16 @@ struct DiluDev {
     int W = 0, M = 0, nLoS = 0, nUpS = 0;
     size_t smem = 0;   // > 0: shared-memory sweeps with this many bytes per CTA
     int threads = 0;   // their CTA size: the widest level rounded up to whole warps (cheap barriers)
+    // pipelined parts (dilupart.cuh): used otherwise; their entries are sLo* / sUp* above
+    DBuf<DiluPart> parts;
+    DBuf<DiluStep> steps;
+    DBuf<int32_t> loRemote, upRemote, loMail, upMail;
+    DBuf<DiluMail> loBox, upBox;
+    DBuf<DiluPartSync> psync;
+    DBuf<double> ws;
+    int nParts = 0, maxRemote = 0;
+    bool local = false;  // each part's vector in shared memory
+    size_t partSmem = 0;
 };
 
 
@@ -409,7 +420,7 @@ void DeviceBatch::endEmbedding() {
     tl_capturing = false;
 }
 
-bool DeviceBatch::embeddable() const { return useGraphs_ && !(dilu_ && dilu_->G > 1); }
+bool DeviceBatch::embeddable() const { return useGraphs_ && !(dilu_ && dilu_->groupSweeps); }
 
 bool DeviceBatch::levelScheduleInSharedMemory(const vlm_solver_ctrl& ctrl) {
     PrecondKind pk = parsePrecond(ctrl.preconditioner);
@@ -1310,39 +1321,91 @@ void DeviceBatch::recordBicgIterT(PrecondKind pk, SmootherKind sm, bool f32) {
 }
 
 // ====================================================================== level-scheduled paths
+// The pipelined schedule.  A part gets about kPartWidth rows of a full level (one per thread, with
+// room for uneven cuts), and no more rows than its vector's share of shared memory: more parts would
+// lengthen the start-up of the pipeline, fewer would split levels into several steps.  Systems that
+// would need more parts than SMs that way keep their vectors in global memory.
+void DeviceBatch::planDiluParts(DiluDev& D, const DiluPlan& P, int sms) {
+    constexpr int kPartWidth = 192;
+    constexpr size_t kSmemMax = 220 * 1024;
+    const int M = std::max(1, std::min(P.maxEnt, kPartEnt));
+    DiluParts R;
+    auto plan = [&](int maxSlots, int W, bool one) {
+        std::vector<int> np(P.sys.size(), 1);
+        int64_t total = 0;
+        for (size_t b = 0; b < P.sys.size(); ++b) {
+            const DiluSys& ds = P.sys[b];
+            int width = 0;
+            for (int t = 0; t < ds.nLev; ++t)
+                width = std::max(width, P.levPtr[ds.levBegin + t + 1] - P.levPtr[ds.levBegin + t]);
+            if (!one) np[b] = std::max((width + kPartWidth - 1) / kPartWidth, maxSlots ? (ds.rowCount + maxSlots - 1) / maxSlots : 1);
+            total += np[b];
+        }
+        if (maxSlots && P.sys.size() == 1 && total > sms) return false;
+        if (!maxSlots && P.sys.size() == 1) np[0] = std::min(np[0], sms);
+        R = buildDiluParts(P, plan_, np, W);
+        D.partSmem = part_smem(maxSlots ? R.maxSlots : 0, R.maxWidth, M, R.maxRemote);
+        return D.partSmem <= kSmemMax;
+    };
+    const int slots = int((kSmemMax - part_smem(0, kPartThreads, M, 2 * kPartThreads)) / sizeof(double));
+    D.local = slots > 0 && plan(slots, kPartThreads, false);
+    if (!D.local && !plan(0, kPartThreads, false) && !plan(0, 32, true))
+        throw Error(VLM_ERR_UNSUPPORTED, "internal: level schedule does not fit");
+    static const bool raised = [] {
+        for (auto k : {k_dilu_part<kPartFactor, true>, k_dilu_part<kPartForward, true>, k_dilu_part<kPartBackward, true>,
+                       k_dilu_part<kPartFactor, false>, k_dilu_part<kPartForward, false>,
+                       k_dilu_part<kPartBackward, false>})
+            VLM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemMax)));
+        return true;
+    }();
+    (void)raised;
+    cudaStream_t s = stream_;
+    D.W = R.maxWidth;
+    D.M = M;
+    D.maxRemote = R.maxRemote;
+    D.nParts = int(R.parts.size());
+    D.parts.upload(R.parts, s);
+    D.steps.upload(R.steps, s);
+    D.slotRow.upload(R.slotRow, s);
+    D.sLoCol.upload(R.loCol, s);
+    D.sLoFace.upload(R.loFace, s);
+    D.sUpCol.upload(R.upCol, s);
+    D.sUpFace.upload(R.upFace, s);
+    D.nLoS = int(R.loCol.size());
+    D.nUpS = int(R.upCol.size());
+    D.loRemote.upload(R.loRemote, s);
+    D.upRemote.upload(R.upRemote, s);
+    D.loMail.upload(R.loMail, s);
+    D.upMail.upload(R.upMail, s);
+    D.loBox.resize(size_t(std::max(R.nLoMail, 1)));
+    D.loBox.zero(s);
+    D.upBox.resize(size_t(std::max(R.nUpMail, 1)));
+    D.upBox.zero(s);
+    D.psync.resize(1);
+    D.psync.zero(s);
+    D.rDs.resize(std::max<size_t>(R.slotRow.size(), 1));
+    D.ws.resize(std::max<size_t>(R.slotRow.size(), 1));
+    VLM_CUDA(cudaStreamSynchronize(s));  // R is a local
+}
+
 void DeviceBatch::ensureDilu() {
     if (dilu_) return;
     const DiluPlan P = buildDiluPlan(topo_, plan_);
     auto D = std::make_unique<DiluDev>();
     cudaStream_t s = stream_;
-    D->loPtr.upload(P.loPtr, s);
-    D->loCol.upload(P.loCol, s);
-    D->loFace.upload(P.loFace, s);
-    D->upPtr.upload(P.upPtr, s);
-    D->upCol.upload(P.upCol, s);
-    D->upFace.upload(P.upFace, s);
     D->levPtr.upload(P.levPtr, s);
     D->levRows.upload(P.levRows, s);
     D->sys.upload(P.sys, s);
-    D->nFaces = int(P.loCol.size());
-    const size_t nf = size_t(std::max(D->nFaces, 1));
-    D->loAul.resize(nf);
-    D->loAlu.resize(nf);
-    D->upAlu.resize(nf);
-    D->rD.resize(size_t(L_[0].nrows));
     D->groups = int(P.sys.size());
-    // one CTA per system; a single wide system gets a co-resident group of CTAs
+    int dev = 0, sms = 0;
+    VLM_CUDA(cudaGetDevice(&dev));
+    VLM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    // Gauss-Seidel: one CTA per system; a single wide system gets a co-resident group of CTAs
     D->G = 1;
     if (D->groups == 1 && P.maxWidth > 2 * kDiluThreads) {
-        int dev = 0, sms = 0, per = 0;
-        VLM_CUDA(cudaGetDevice(&dev));
-        VLM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        VLM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_dilu_apply, kDiluThreads, 0));
-        int perF = 0, perG = 0;
-        VLM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perF, k_dilu_factor, kDiluThreads, 0));
-        VLM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perG, k_gs_sweep, kDiluThreads, 0));
-        const int resident = sms * std::max(1, std::min(per, std::min(perF, perG)));
-        D->G = std::max(1, std::min({(P.maxWidth + kDiluThreads - 1) / kDiluThreads, resident, sms}));
+        int per = 0;
+        VLM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_gs_sweep, kDiluThreads, 0));
+        D->G = std::max(1, std::min({(P.maxWidth + kDiluThreads - 1) / kDiluThreads, sms * std::max(1, per), sms}));
     }
     // shared-memory sweeps: one CTA per system, every level at most one row per thread, the vector
     // of the largest system within the opt-in shared memory
@@ -1372,11 +1435,13 @@ void DeviceBatch::ensureDilu() {
         D->sUpFace.upload(P.sUpFace, s);
         D->nLoS = int(P.sLoCol.size());
         D->nUpS = int(P.sUpCol.size());
-        D->prod.resize(size_t(std::max(D->nLoS, 1)));
-        D->coefLo.resize(size_t(std::max(D->nLoS, 1)));
-        D->coefUp.resize(size_t(std::max(D->nUpS, 1)));
         D->rDs.resize(std::max<size_t>(P.slotRow.size(), 1));
+    } else {
+        planDiluParts(*D, P, sms);
     }
+    D->prod.resize(size_t(std::max(D->nLoS, 1)));
+    D->coefLo.resize(size_t(std::max(D->nLoS, 1)));
+    D->coefUp.resize(size_t(std::max(D->nUpS, 1)));
     D->bars.resize(size_t(D->groups));
     D->bars.zero(s);
     D->err.resize(1);
@@ -1406,10 +1471,10 @@ void launchLevels(void (*kernel)(Exp...), int groups, int G, cudaStream_t s, Act
 void DeviceBatch::diluFactor(const double* upper, const double* lower) {
     DiluDev& Dd = *dilu_;
     cudaStream_t s = stream_;
+    VLM_LAUNCH(k_dilu_stream_values, nblk(std::max(1, Dd.nLoS + Dd.nUpS)), 256, s, Dd.nLoS, Dd.nUpS,
+               (const int32_t*)Dd.sLoCol.get(), (const int32_t*)Dd.sLoFace.get(), (const int32_t*)Dd.sUpCol.get(),
+               (const int32_t*)Dd.sUpFace.get(), upper, lower, Dd.prod.get(), Dd.coefLo.get(), Dd.coefUp.get());
     if (Dd.smem) {
-        VLM_LAUNCH(k_dilu_stream_values, nblk(std::max(1, Dd.nLoS + Dd.nUpS)), 256, s, Dd.nLoS, Dd.nUpS,
-                   (const int32_t*)Dd.sLoCol.get(), (const int32_t*)Dd.sLoFace.get(), (const int32_t*)Dd.sUpCol.get(),
-                   (const int32_t*)Dd.sUpFace.get(), upper, lower, Dd.prod.get(), Dd.coefLo.get(), Dd.coefUp.get());
         k_dilu_factor_stream<<<Dd.groups, Dd.threads, Dd.smem, s>>>(Dd.sys.get(), Dd.lev.get(), Dd.W, Dd.M,
                                                                       Dd.slotRow.get(), Dd.sLoCol.get(), Dd.prod.get(),
                                                                       L_[0].diag.get(), Dd.rDs.get());
@@ -1417,12 +1482,24 @@ void DeviceBatch::diluFactor(const double* upper, const double* lower) {
         ++tl_launches;
         return;
     }
-    VLM_LAUNCH(k_dilu_values, nblk(Dd.nFaces), 256, s, Dd.nFaces, (const int32_t*)Dd.loFace.get(),
-               (const int32_t*)Dd.upFace.get(), upper, lower, Dd.loAul.get(), Dd.loAlu.get(), Dd.upAlu.get());
-    launchLevels(k_dilu_factor, Dd.groups, Dd.G, s, (const DiluSys*)Dd.sys.get(), Dd.G, (const int32_t*)Dd.levPtr.get(),
-                 (const int32_t*)Dd.levRows.get(), (const int32_t*)Dd.loPtr.get(), (const int32_t*)Dd.loCol.get(),
-                 (const double*)Dd.loAlu.get(), (const double*)Dd.loAul.get(), (const double*)L_[0].diag.get(),
-                 Dd.rD.get(), Dd.bars.get(), Dd.err.get());
+    launchDiluPart<kPartFactor>(L_[0].diag.get(), nullptr, nullptr);
+}
+
+// One factorisation or sweep over the pipelined parts; st: skip the systems that are done.
+template <int KIND>
+void DeviceBatch::launchDiluPart(const double* src, double* w, const SysState* st) {
+    DiluDev& D = *dilu_;
+    constexpr bool back = KIND == kPartBackward;
+    const DiluPartArgs A{D.parts.get(), D.steps.get(), D.nParts, D.W, D.M, D.maxRemote, D.slotRow.get(),
+                         back ? D.sUpCol.get() : D.sLoCol.get(), back ? D.upRemote.get() : D.loRemote.get(),
+                         back ? D.upMail.get() : D.loMail.get(),
+                         KIND == kPartFactor ? D.prod.get() : back ? D.coefUp.get() : D.coefLo.get(),
+                         back ? D.upBox.get() : D.loBox.get(), D.rDs.get(), D.ws.get(), src, w, D.psync.get(),
+                         D.err.get(), st, int(kFlagDone)};
+    if (D.local)
+        VLM_LAUNCH_SMEM((k_dilu_part<KIND, true>), D.nParts, kPartThreads, D.partSmem, stream_, A);
+    else
+        VLM_LAUNCH_SMEM((k_dilu_part<KIND, false>), D.nParts, kPartThreads, D.partSmem, stream_, A);
 }
 
 void DeviceBatch::clearLevelError() {
@@ -1454,11 +1531,8 @@ void DeviceBatch::recordDiluApply(const double* r, double* w) {
         ++tl_launches;
         return;
     }
-    launchLevels(k_dilu_apply, D.groups, D.G, stream_, (const DiluSys*)D.sys.get(), D.G, (const int32_t*)D.levPtr.get(),
-                 (const int32_t*)D.levRows.get(), (const int32_t*)D.loPtr.get(), (const int32_t*)D.loCol.get(),
-                 (const double*)D.loAul.get(), (const int32_t*)D.upPtr.get(), (const int32_t*)D.upCol.get(),
-                 (const double*)D.upAlu.get(), (const double*)D.rD.get(), r, w, D.bars.get(), D.err.get(),
-                 (const SysState*)st_.get(), int(kFlagDone));
+    launchDiluPart<kPartForward>(r, nullptr, st_.get());
+    launchDiluPart<kPartBackward>(nullptr, w, st_.get());
 }
 
 // Gauss-Seidel / symmetric Gauss-Seidel / Jacobi: nSweeps sweeps, then the residual and the
@@ -1484,6 +1558,7 @@ void DeviceBatch::recordRelaxIterT(const SolveKey& key) {
             VLM_LAUNCH(k_copy_rows<double>, nb, kRowsPerCta, s, ch, w_.get(), x_.get(), st_.get(), kFlagDone);
         } else {
             DiluDev& D = *dilu_;
+            D.groupSweeps = D.groupSweeps || D.G > 1;
             for (int dir = 0; dir < (key.solver == SolverKind::SymGaussSeidel ? 2 : 1); ++dir)
                 launchLevels(k_gs_sweep, D.groups, D.G, s, (const DiluSys*)D.sys.get(), D.G,
                              (const int32_t*)D.levPtr.get(), (const int32_t*)D.levRows.get(), D0.sell(),

@@ -69,6 +69,7 @@ struct SolveKey {
     }
 };
 
+struct DiluPlan;
 struct DiluDev;  // device copy of the DIC/DILU / Gauss-Seidel level schedule (solver.cu)
 
 struct GraphExec {
@@ -219,6 +220,8 @@ private:
     void planTail();
     void buildChunkLists();
     void ensureDilu();
+    void planDiluParts(DiluDev& D, const DiluPlan& P, int sms);
+    template <int KIND> void launchDiluPart(const double* src, double* w, const SysState* st);
     void recordDiluApply(const double* r, double* w);
     void diluFactor(const double* upper, const double* lower);
     void checkLevelError();
