@@ -220,4 +220,59 @@ DiluParts buildDiluParts(const DiluPlan& D, const BatchPlan& P, const std::vecto
     return R;
 }
 
+bool buildDiluRecords(const DiluParts& R, DiluRecords& out) {
+    const size_t ns = R.slotRow.size();
+    out = DiluRecords{};
+    if (R.nLoMail >= (1 << 21) || R.nUpMail >= (1 << 21)) return false;
+    out.steps.resize(R.steps.size());
+    for (int dir = 0; dir < 2; ++dir) {
+        const std::vector<int32_t>&col = dir ? R.upCol : R.loCol, &face = dir ? R.upFace : R.loFace,
+                         &mail = dir ? R.upMail : R.loMail;
+        std::vector<int32_t>&oc = dir ? out.upCol : out.loCol, &of = dir ? out.upFace : out.loFace;
+        oc.assign(4 * ns, -1);
+        of.assign(4 * ns, DiluRecords::kNoFace);
+        for (const DiluPart& P : R.parts) {
+            out.maxSteps = std::max(out.maxSteps, P.nSteps);
+            for (int i = 0; i < P.nSteps; ++i) {
+                const DiluStep& S = R.steps[size_t(P.stepBegin + i)];
+                DiluRecStep& T = out.steps[size_t(P.stepBegin + i)];
+                T.s0 = S.s0;
+                T.width = S.width;
+                T.rlo = S.rlo;
+                T.nrlo = S.nrlo;
+                T.rup = S.rup;
+                T.nrup = S.nrup;
+                const int e0 = dir ? S.up : S.lo, m = dir ? S.mup : S.mlo;
+                if (m > 6) return false;
+                const int ext0 = int(oc.size() / 4);
+                int nExt = 0;
+                for (int q = 0; q < S.width; ++q) {
+                    const size_t slot = size_t(S.s0 + q);
+                    int n = 0;
+                    while (n < m && col[size_t(e0 + n * S.width + q)] != -1) ++n;
+                    size_t ext = 0;
+                    if (n > 3) {
+                        ext = size_t(ext0 + nExt++);
+                        oc.resize(4 * (ext + 1), -1);
+                        of.resize(4 * (ext + 1), DiluRecords::kNoFace);
+                    }
+                    for (int j = 0; j < n; ++j) {
+                        const size_t at = j < 3 ? 4 * slot + size_t(j) : 4 * ext + size_t(j - 3);
+                        const int l = col[size_t(e0 + j * S.width + q)];
+                        oc[at] = l >= 0 ? l : P.nSlots + (i & 1) * R.maxRemote + (-2 - l);
+                        of[at] = face[size_t(e0 + j * S.width + q)];
+                    }
+                    oc[4 * slot + 3] = ((mail[slot] + 1) << 9) | (n > 3 ? int(ext) - ext0 + 1 : 0);
+                }
+                if (nExt >= 511) return false;
+                (dir ? T.extUp : T.extLo) = ext0;
+                (dir ? T.nExtUp : T.nExtLo) = nExt;
+                out.maxExt = std::max(out.maxExt, nExt);
+            }
+        }
+        (dir ? out.nUp : out.nLo) = int(oc.size() / 4);
+    }
+    return true;
+}
+
 }  // namespace vlm

@@ -84,6 +84,26 @@ struct DiluParts {
     int maxSlots = 0, maxWidth = 0, maxRemote = 0;
 };
 
+// The parts' entries as 16-byte records for rows of at most six lower and six upper neighbours (box
+// meshes): record [slot] holds the first three columns and, in its fourth word, 1 + mailbox << 9 | 1 + the
+// extension's place in the step (0: none); the extensions of a step's rows with more entries follow at
+// extLo / extUp of the step.  Columns index the part's vector in shared memory: its slots, then two
+// buffers of maxRemote remote values (step parity); -1: no entry.  faces: as DiluPlan's, kNoFace: none.
+struct DiluRecStep {
+    int s0, width, rlo, nrlo, rup, nrup, extLo, nExtLo, extUp, nExtUp;
+};
+
+struct DiluRecords {
+    static constexpr int32_t kNoFace = 0x7fffffff;
+    std::vector<DiluRecStep> steps;
+    std::vector<int32_t> loCol, upCol, loFace, upFace;  // four words per record
+    int nLo = 0, nUp = 0;                               // records (slots, then extensions)
+    int maxExt = 0, maxSteps = 0;
+};
+
+// False when a row has more than six entries in a direction or a word overflows.
+bool buildDiluRecords(const DiluParts& R, DiluRecords& out);
+
 // nParts[b]: parts of the system at batch position b (at least 1).
 DiluParts buildDiluParts(const DiluPlan& D, const BatchPlan& P, const std::vector<int>& nParts, int maxWidth);
 

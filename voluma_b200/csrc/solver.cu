@@ -48,6 +48,12 @@ struct DiluDev {
     int nParts = 0, maxRemote = 0;
     bool local = false;  // each part's vector in shared memory
     size_t partSmem = 0;
+    int stepsLocal = 0;
+    // packed records (k_dilu_pipe), where the rows allow them; coefficients in prod / coefLo / coefUp
+    bool records = false;
+    DBuf<DiluRecStep> recSteps;
+    DBuf<int32_t> recLoCol, recUpCol, recLoFace, recUpFace;
+    int nRecLo = 0, nRecUp = 0, maxExt = 0, ring = 0;
 };
 
 
@@ -1323,13 +1329,16 @@ void DeviceBatch::recordBicgIterT(PrecondKind pk, SmootherKind sm, bool f32) {
 // ====================================================================== level-scheduled paths
 // The pipelined schedule.  A part gets about kPartWidth rows of a full level (one per thread, with
 // room for uneven cuts), and no more rows than its vector's share of shared memory: more parts would
-// lengthen the start-up of the pipeline, fewer would split levels into several steps.  Systems that
-// would need more parts than SMs that way keep their vectors in global memory.
+// lengthen the start-up of the pipeline, fewer would split levels into several steps.  Packed records
+// where every row has at most six entries per direction and the parts' vectors fit with a ring of
+// three stages at least; else the general kernel, with its vectors in global memory where a system
+// would need more parts than SMs.
 void DeviceBatch::planDiluParts(DiluDev& D, const DiluPlan& P, int sms) {
     constexpr int kPartWidth = 192;
     constexpr size_t kSmemMax = 220 * 1024;
-    const int M = std::max(1, std::min(P.maxEnt, kPartEnt));
     DiluParts R;
+    DiluRecords C;
+    // the parts for at most maxSlots slots each (0: any) and steps of at most W rows; one: a part per system
     auto plan = [&](int maxSlots, int W, bool one) {
         std::vector<int> np(P.sys.size(), 1);
         int64_t total = 0;
@@ -1344,17 +1353,54 @@ void DeviceBatch::planDiluParts(DiluDev& D, const DiluPlan& P, int sms) {
         if (maxSlots && P.sys.size() == 1 && total > sms) return false;
         if (!maxSlots && P.sys.size() == 1) np[0] = std::min(np[0], sms);
         R = buildDiluParts(P, plan_, np, W);
-        D.partSmem = part_smem(maxSlots ? R.maxSlots : 0, R.maxWidth, M, R.maxRemote);
-        return D.partSmem <= kSmemMax;
+        return true;
     };
-    const int slots = int((kSmemMax - part_smem(0, kPartThreads, M, 2 * kPartThreads)) / sizeof(double));
-    D.local = slots > 0 && plan(slots, kPartThreads, false);
-    if (!D.local && !plan(0, kPartThreads, false) && !plan(0, 32, true))
-        throw Error(VLM_ERR_UNSUPPORTED, "internal: level schedule does not fit");
+    auto slotsFor = [&](size_t fixed) { return fixed < kSmemMax ? int((kSmemMax - fixed) / sizeof(double)) : 0; };
+    if (P.maxEnt <= 6) {
+        // extensions, remote entries and steps are known once a plan exists: a first guess, then its figures
+        int E = P.maxEnt > 3 ? 64 : 0, rem = kPartThreads, steps = 512;
+        for (int ring = 5; ring >= 3 && !D.records; --ring)
+            for (int guess = 0; guess < 2; ++guess) {
+                const int slots = slotsFor(pipe_smem(0, kPartThreads, E, rem, ring, steps));
+                if (slots < 1 || !plan(slots, kPartThreads, false)) break;
+                if (!buildDiluRecords(R, C)) {
+                    ring = 0;
+                    break;
+                }
+                D.partSmem = pipe_smem(R.maxSlots, R.maxWidth, C.maxExt, R.maxRemote, ring, C.maxSteps);
+                if (D.partSmem <= kSmemMax) {
+                    D.records = true;
+                    D.ring = ring;
+                    break;
+                }
+                E = C.maxExt;
+                rem = R.maxRemote;
+                steps = C.maxSteps;
+            }
+    }
+    const int M = std::max(1, std::min(P.maxEnt, kPartEnt));
+    if (!D.records) {
+        auto fits = [&](int localSlots) {
+            int most = 0;
+            for (const DiluPart& q : R.parts) most = std::max(most, q.nSteps);
+            for (int steps : {most, 0}) {
+                D.stepsLocal = steps;
+                D.partSmem = part_smem(localSlots, R.maxWidth, M, R.maxRemote, steps);
+                if (D.partSmem <= kSmemMax) return true;
+            }
+            return false;
+        };
+        const int slots = slotsFor(part_smem(0, kPartThreads, M, 2 * kPartThreads, 512));
+        D.local = slots > 0 && plan(slots, kPartThreads, false) && fits(R.maxSlots);
+        if (!D.local && !(plan(0, kPartThreads, false) && fits(0)) && !(plan(0, 32, true) && fits(0)))
+            throw Error(VLM_ERR_UNSUPPORTED, "internal: level schedule does not fit");
+    }
     static const bool raised = [] {
         for (auto k : {k_dilu_part<kPartFactor, true>, k_dilu_part<kPartForward, true>, k_dilu_part<kPartBackward, true>,
                        k_dilu_part<kPartFactor, false>, k_dilu_part<kPartForward, false>,
                        k_dilu_part<kPartBackward, false>})
+            VLM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemMax)));
+        for (auto k : {k_dilu_pipe<kPartFactor>, k_dilu_pipe<kPartForward>, k_dilu_pipe<kPartBackward>})
             VLM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemMax)));
         return true;
     }();
@@ -1365,27 +1411,38 @@ void DeviceBatch::planDiluParts(DiluDev& D, const DiluPlan& P, int sms) {
     D.maxRemote = R.maxRemote;
     D.nParts = int(R.parts.size());
     D.parts.upload(R.parts, s);
-    D.steps.upload(R.steps, s);
     D.slotRow.upload(R.slotRow, s);
-    D.sLoCol.upload(R.loCol, s);
-    D.sLoFace.upload(R.loFace, s);
-    D.sUpCol.upload(R.upCol, s);
-    D.sUpFace.upload(R.upFace, s);
-    D.nLoS = int(R.loCol.size());
-    D.nUpS = int(R.upCol.size());
     D.loRemote.upload(R.loRemote, s);
     D.upRemote.upload(R.upRemote, s);
-    D.loMail.upload(R.loMail, s);
-    D.upMail.upload(R.upMail, s);
     D.loBox.resize(size_t(std::max(R.nLoMail, 1)));
     D.loBox.zero(s);
     D.upBox.resize(size_t(std::max(R.nUpMail, 1)));
     D.upBox.zero(s);
     D.psync.resize(1);
     D.psync.zero(s);
-    D.rDs.resize(std::max<size_t>(R.slotRow.size(), 1));
     D.ws.resize(std::max<size_t>(R.slotRow.size(), 1));
-    VLM_CUDA(cudaStreamSynchronize(s));  // R is a local
+    if (D.records) {
+        D.nRecLo = C.nLo;
+        D.nRecUp = C.nUp;
+        D.maxExt = C.maxExt;
+        D.recSteps.upload(C.steps, s);
+        D.recLoCol.upload(C.loCol, s);
+        D.recUpCol.upload(C.upCol, s);
+        D.recLoFace.upload(C.loFace, s);
+        D.recUpFace.upload(C.upFace, s);
+    } else {
+        D.steps.upload(R.steps, s);
+        D.sLoCol.upload(R.loCol, s);
+        D.sLoFace.upload(R.loFace, s);
+        D.sUpCol.upload(R.upCol, s);
+        D.sUpFace.upload(R.upFace, s);
+        D.nLoS = int(R.loCol.size());
+        D.nUpS = int(R.upCol.size());
+        D.loMail.upload(R.loMail, s);
+        D.upMail.upload(R.upMail, s);
+        D.rDs.resize(std::max<size_t>(R.slotRow.size(), 1));
+    }
+    VLM_CUDA(cudaStreamSynchronize(s));  // R and C are locals
 }
 
 void DeviceBatch::ensureDilu() {
@@ -1439,9 +1496,11 @@ void DeviceBatch::ensureDilu() {
     } else {
         planDiluParts(*D, P, sms);
     }
-    D->prod.resize(size_t(std::max(D->nLoS, 1)));
-    D->coefLo.resize(size_t(std::max(D->nLoS, 1)));
-    D->coefUp.resize(size_t(std::max(D->nUpS, 1)));
+    const size_t nLo = D->records ? 4 * size_t(D->nRecLo) : size_t(std::max(D->nLoS, 1));
+    const size_t nUp = D->records ? 4 * size_t(D->nRecUp) : size_t(std::max(D->nUpS, 1));
+    D->prod.resize(nLo);
+    D->coefLo.resize(nLo);
+    D->coefUp.resize(nUp);
     D->bars.resize(size_t(D->groups));
     D->bars.zero(s);
     D->err.resize(1);
@@ -1471,6 +1530,13 @@ void launchLevels(void (*kernel)(Exp...), int groups, int G, cudaStream_t s, Act
 void DeviceBatch::diluFactor(const double* upper, const double* lower) {
     DiluDev& Dd = *dilu_;
     cudaStream_t s = stream_;
+    if (Dd.records) {
+        VLM_LAUNCH(k_dilu_record_values, nblk(Dd.nRecLo + Dd.nRecUp), 256, s, Dd.nRecLo, Dd.nRecUp,
+                   (const int4*)Dd.recLoFace.get(), (const int4*)Dd.recUpFace.get(), upper, lower, Dd.prod.get(),
+                   Dd.coefLo.get(), Dd.coefUp.get());
+        launchDiluPart<kPartFactor>(L_[0].diag.get(), nullptr, nullptr);
+        return;
+    }
     VLM_LAUNCH(k_dilu_stream_values, nblk(std::max(1, Dd.nLoS + Dd.nUpS)), 256, s, Dd.nLoS, Dd.nUpS,
                (const int32_t*)Dd.sLoCol.get(), (const int32_t*)Dd.sLoFace.get(), (const int32_t*)Dd.sUpCol.get(),
                (const int32_t*)Dd.sUpFace.get(), upper, lower, Dd.prod.get(), Dd.coefLo.get(), Dd.coefUp.get());
@@ -1490,7 +1556,17 @@ template <int KIND>
 void DeviceBatch::launchDiluPart(const double* src, double* w, const SysState* st) {
     DiluDev& D = *dilu_;
     constexpr bool back = KIND == kPartBackward;
-    const DiluPartArgs A{D.parts.get(), D.steps.get(), D.nParts, D.W, D.M, D.maxRemote, D.slotRow.get(),
+    if (D.records) {
+        const DiluPipeArgs A{D.parts.get(), D.recSteps.get(), D.nParts, D.W, D.maxExt, D.maxRemote, D.ring,
+                             D.slotRow.get(), (const int4*)(back ? D.recUpCol.get() : D.recLoCol.get()),
+                             KIND == kPartFactor ? D.prod.get() : back ? D.coefUp.get() : D.coefLo.get(),
+                             back ? D.upRemote.get() : D.loRemote.get(), back ? D.upBox.get() : D.loBox.get(),
+                             D.coefLo.get(), D.coefUp.get(), D.ws.get(), src, w, D.psync.get(), D.err.get(), st,
+                             int(kFlagDone)};
+        VLM_LAUNCH_SMEM(k_dilu_pipe<KIND>, D.nParts, kPartThreads, D.partSmem, stream_, A);
+        return;
+    }
+    const DiluPartArgs A{D.parts.get(), D.steps.get(), D.nParts, D.W, D.M, D.maxRemote, D.stepsLocal, D.slotRow.get(),
                          back ? D.sUpCol.get() : D.sLoCol.get(), back ? D.upRemote.get() : D.loRemote.get(),
                          back ? D.upMail.get() : D.loMail.get(),
                          KIND == kPartFactor ? D.prod.get() : back ? D.coefUp.get() : D.coefLo.get(),
