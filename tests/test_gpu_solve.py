@@ -84,6 +84,30 @@ def test_exact_sum_bitwise():
     assert np.isnan(vb.exact_sum([1.0, np.nan])) and vb.exact_sum([np.inf, 2.0]) == np.inf
 
 
+@pytest.mark.parametrize("n", [1, 31, 33, 255, 257, 4097])
+def test_exact_sum_bin_positions_bitwise(n):
+    """Neighbouring values far apart in magnitude (every lane of a warp in other bins), subnormal ones,
+    a negative total, and totals that cancel to the last bin."""
+    rng = np.random.default_rng(n)
+    v = rng.standard_normal(n) * 10.0 ** rng.uniform(-320, 300, n)
+    for a in (v, -np.abs(v), np.concatenate([v, -v]), np.concatenate([v, [5e-324], -v])):
+        assert vb.exact_sum(a) == ro.exact_sum(a)
+
+
+@pytest.mark.parametrize("spread", [0.0, 3.0, 60.0])
+def test_reproducible_sums_of_spread_rows_bitwise(spread):
+    """The solve's own exact sums, four rows a thread: rows whose magnitudes change the bin position
+    from one to the next."""
+    g, m = device_mesh("periodic24")
+    n = g["b"].size
+    b = g["b"] * 10.0 ** np.random.default_rng(5).uniform(-spread, spread, n)
+    x = np.zeros(n)
+    p = vb.solve_ldu(m, g["diag"], g["upper"], None, b, x, ctrl(reproducible=True, relTol=0.0, maxIter=4))
+    xo, po = ro.solve(g, g["diag"], g["upper"], None, b, np.zeros(n), "PCG", "diagonal", 0.0, 0.0, 4, exact=True)
+    assert np.array_equal(x, xo) and p.iterations == po["iterations"]
+    assert p.finalResidual == po["finalResidual"] and p.initialResidual == po["initialResidual"]
+
+
 @pytest.mark.parametrize("name", golden_names())
 def test_pcg_diagonal_reproducible_bitwise(name):
     """CFD_REPRODUCIBLE mode: exact sums + the reference's operation order -> the reference's
