@@ -415,6 +415,54 @@ def test_shared_memory_tail_matches_global_tail(name, precision, monkeypatch):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("shape,periodic", [((5, 5, 5), (1, 1, 1)), ((9, 7, 5), (1, 0, 0)), ((20, 20, 20), (0, 0, 0)),
+                                            ((64, 64, 1), (0, 0, 0)), ((32, 31, 19), (0, 1, 0))])
+@pytest.mark.parametrize("smoother", ["mcgs-jacobi", "jacobi"])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_cluster_tail_default_start_matches_global_tail(shape, periodic, smoother, precision, monkeypatch):
+    """Where the shared-memory tail starts by itself (level 0 with two or more colours, a coarse level,
+    the last cluster's slices not full): the solution of the global-memory tail bit for bit."""
+    M = vm.box_mesh(shape, periodic=periodic, two_d=shape[2] == 1)
+    d, up = vm.poisson_matrix(M)
+    b = np.random.default_rng(4).standard_normal(M["n_cells"])
+    b -= b.mean()
+    monkeypatch.setenv("VLM_TUNE", "0")
+    out = []
+    for smem in ("0", "1"):
+        monkeypatch.setenv("VLM_TAIL_SMEM", smem)
+        m = vb.Mesh.from_arrays(M)
+        x = np.zeros(M["n_cells"])
+        p = vb.solve_ldu(m, d, up, None, b, x, ctrl(preconditioner="GAMG", smoother=smoother, precision=precision))
+        out.append((x, p.iterations))
+        m.close()
+    assert out[0][1] == out[1][1] and np.array_equal(out[0][0], out[1][0])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("systems", [3, 20, 40, 80])
+def test_tail_cluster_widths_of_a_batch_match_solo(systems):
+    """More systems take narrower clusters (8, 4, 2 CTAs, one): each system's solution is its own."""
+    shapes = [(6 + q % 5, 7 + q % 3, 5 + q % 4) for q in range(systems)]
+    meshes = [vm.box_mesh(s) for s in shapes]
+    rng = np.random.default_rng(8)
+    data = []
+    for M in meshes:
+        d, up = vm.poisson_matrix(M)
+        b = rng.standard_normal(M["n_cells"])
+        data.append((d, up, b - b.mean()))
+    B = vb.Mesh.batch(meshes)
+    c = ctrl(preconditioner="GAMG")
+    x = np.zeros(B.n_cells)
+    vb.solve_ldu(B, *(np.concatenate([q[k] for q in data]) for k in (0, 1)), None,
+                 np.concatenate([q[2] for q in data]), x, c)
+    base = np.cumsum([0] + [M["n_cells"] for M in meshes])
+    for q in range(0, systems, 7):
+        xs = np.zeros(meshes[q]["n_cells"])
+        vb.solve_ldu(vb.Mesh.from_arrays(meshes[q]), data[q][0], data[q][1], None, data[q][2], xs, c)
+        assert np.array_equal(x[base[q]:base[q + 1]], xs), q
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("shape,periodic", [((32, 16, 8), (1, 1, 1)), ((64, 16, 6), (0, 0, 0)),
                                             ((32, 32, 12), (1, 0, 1)), ((64, 24, 4), (1, 1, 1))])
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])

@@ -80,10 +80,11 @@ struct TailSys {
     int grpStart[4], grpCount[4];
 };
 
-// One system's coarse tail in shared memory (k_vcycle_tail_smem): the Jacobi levels first..coarsest-1
-// as ELL rows with 16-bit local columns, the coarsest level's dense inverse, and every level's
-// vectors.  t* are element offsets into the T region of shared memory (the value image, then the
-// vectors), u* into the uint16 region (structure image).
+// One CTA's part of a system's coarse tail in shared memory (k_vcycle_tail_parts): its 32-row slices
+// (slice s of a level belongs to CTA s mod cluster) of the levels first..coarsest-1, its rows of the
+// coarsest level's dense inverse, and every level's vectors.  t* are element offsets into the T
+// region of shared memory (vectors, at the same places in every CTA of the cluster; then the value
+// image), u* into the uint16 region (structure image).
 #ifdef __CUDACC__
 #define VLM_HD __host__ __device__
 #else
@@ -91,21 +92,24 @@ struct TailSys {
 #endif
 VLM_HD constexpr size_t tail_align16(size_t b) { return (b + 15) & ~size_t(15); }
 
-// Shared-memory bytes of one system's tail: the T region, the coarsest inverse (doubles), the
+// Shared-memory bytes of one part: the T region, the rows of the coarsest inverse (doubles), the
 // uint16 region, each starting on a 16-byte boundary.
-VLM_HD inline size_t tail_smem_bytes(size_t tsize, int tCount, int nc, int strCount) {
-    return tail_align16(size_t(tCount) * tsize) + tail_align16(size_t(nc) * nc * sizeof(double)) +
+VLM_HD inline size_t tail_smem_bytes(size_t tsize, int tCount, int invCount, int strCount) {
+    return tail_align16(size_t(tCount) * tsize) + tail_align16(size_t(invCount) * sizeof(double)) +
            tail_align16(size_t(strCount) * sizeof(uint16_t));
 }
 
-struct TailImg {
+struct TailPart {
     int sys, first, coarsest, nc, invOffset;
-    int valOff, strOff;              // offsets of this system's images in the batch's image buffers
-    int valCount, tCount, strCount;  // value-image T count; T count in shared memory; uint16 count
-    int n[kTailMaxLevels], W[kTailMaxLevels], rowStart[kTailMaxLevels];
-    int tDiag[kTailMaxLevels], tVal[kTailMaxLevels], tR[kTailMaxLevels], tX[kTailMaxLevels], tX2[kTailMaxLevels];
-    int uRlen[kTailMaxLevels], uCol[kTailMaxLevels], uAgg[kTailMaxLevels], uCptr[kTailMaxLevels],
-        uChild[kTailMaxLevels];
+    int valOff, strOff;              // offsets of this part's images in the batch's image buffers
+    int vecCount, valCount, strCount;  // T counts of the vectors and the value image; uint16 count
+    int two, nColours;               // level 0 in the tail: multicolour Gauss-Seidel groups (TailSys)
+    int grpStart[4], grpCount[4];    // rows relative to the system's first
+    int n[kTailMaxLevels], nl[kTailMaxLevels], rowStart[kTailMaxLevels];  // rows; this CTA's rows; first row
+    int tX[kTailMaxLevels], tX2[kTailMaxLevels];  // iterates, a copy in every CTA (coarsest: solution, right-hand side)
+    int tR[kTailMaxLevels], tDiag[kTailMaxLevels], tVal[kTailMaxLevels];  // this CTA's rows only
+    int uRlen[kTailMaxLevels], uSlice[kTailMaxLevels], uCol[kTailMaxLevels], uAgg[kTailMaxLevels],
+        uCptr[kTailMaxLevels], uChild[kTailMaxLevels];
 };
 
 }  // namespace vlm

@@ -301,10 +301,6 @@ __host__ __device__ constexpr size_t pipe_smem(int slots, int W, int E, int maxR
            dilu_align16(size_t(steps) * sizeof(DiluRecStep));
 }
 
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(unsigned(__cvta_generic_to_shared(dst))), "l"(src)
-                 : "memory");
-}
 __device__ __forceinline__ void cp_async_wait_n(int n) {
     switch (n) {  // all but the n newest groups
     case 1: cp_async_wait<1>(); break;

@@ -19,6 +19,7 @@
 #include "krylov.cuh"
 #include "aggl.h"
 #include "solver.h"
+#include "tailpart.cuh"
 #include "tailplan.h"
 
 namespace vlm {
@@ -289,9 +290,9 @@ DeviceBatch::DeviceBatch(const std::vector<SysTopo>& systems, int mergeLevels, c
             D.x.zero(stream_);
         }
         // host-side plan data no longer needed on the device path; the column indices of levels a
-        // shared-memory tail may take (below level 0, every system under 16-bit local indices) stay
-        // for re-planning the tail (setTail)
-        bool tailLevel = k > 0;
+        // shared-memory tail may take (every system under 16-bit local indices) stay for re-planning
+        // the tail (setTail)
+        bool tailLevel = true;
         for (size_t b = 0; tailLevel && b + 1 < P.sysRow.size(); ++b)
             if (P.sysRow[b + 1] - P.sysRow[b] >= 0xffff) tailLevel = false;
         if (!tailLevel) std::vector<int32_t>().swap(P.col);
@@ -334,8 +335,10 @@ void DeviceBatch::buildChunkLists() {
     for (int k = 0; k < int(L_.size()); ++k) {
         const LevelPlan& P = plan_.levels[k];
         DevLevel& D = L_[k];
-        D.headFwd.clear();
-        D.headRev.clear();
+        for (int p = 0; p < 2; ++p) {
+            D.headFwd[p].clear();
+            D.headRev[p].clear();
+        }
         D.fwd.clear();
         D.rev.clear();
         std::vector<Chunk> all;
@@ -346,24 +349,25 @@ void DeviceBatch::buildChunkLists() {
         };
         D.active = add(P.active);
         D.all = add(P.all);
-        if (tailOn_) {
+        for (int p = 0; tailOn_ && p < 2; ++p) {
             // coarse-tail mode: rows still smoothed by per-level launches, and the rows the last
             // of those restrictions writes (systems whose tail starts at or below this level)
+            const std::vector<int>& first = tailFirst_[p];
             std::vector<Chunk> head, in;
             for (const Chunk& c : P.active)
-                if (tailFirst_[c.sys] > k) head.push_back(c);
+                if (first[c.sys] > k) head.push_back(c);
             for (const Chunk& c : P.all)
-                if (k > 0 && tailFirst_[c.sys] >= k) in.push_back(c);
-            D.headActive = add(head);
-            D.headIn = add(in);
+                if (k > 0 && first[c.sys] >= k) in.push_back(c);
+            D.headActive[p] = add(head);
+            D.headIn[p] = add(in);
             for (int t = 0; t < P.nSteps; ++t) {
                 std::vector<Chunk> hf, hr;
                 for (const Chunk& c : P.fwd[t])
-                    if (tailFirst_[c.sys] > k) hf.push_back(c);
+                    if (first[c.sys] > k) hf.push_back(c);
                 for (const Chunk& c : P.rev[t])
-                    if (tailFirst_[c.sys] > k) hr.push_back(c);
-                D.headFwd.push_back(add(hf));
-                D.headRev.push_back(add(hr));
+                    if (first[c.sys] > k) hr.push_back(c);
+                D.headFwd[p].push_back(add(hf));
+                D.headRev[p].push_back(add(hr));
             }
         }
         for (int t = 0; t < P.nSteps; ++t) D.fwd.push_back(add(P.fwd[t]));
@@ -671,10 +675,12 @@ void DeviceBatch::setupMatrix(const double* diag, const double* upper, const dou
     }
     if (tailOn_ && tailSmem_) {
         // the shared-memory tail's value images of this solve's coarse levels
-        const int nv = int(tailCodes_.size());
-        VLM_LAUNCH(k_tail_values<double>, nblk(nv), 256, s, nv, tailCodes_.get(), tail64_.get(), tailVal64_.get());
+        const int n64 = int(tailPart_[0].codes.size()), n32 = int(tailPart_[1].codes.size());
+        VLM_LAUNCH(k_tail_values<double>, nblk(n64), 256, s, n64, tailPart_[0].codes.get(), tail64_.get(),
+                   tailVal64_.get());
         if (mixed && tail32_.size() != 0)
-            VLM_LAUNCH(k_tail_values<float>, nblk(nv), 256, s, nv, tailCodes_.get(), tail32_.get(), tailVal32_.get());
+            VLM_LAUNCH(k_tail_values<float>, nblk(n32), 256, s, n32, tailPart_[1].codes.get(), tail32_.get(),
+                       tailVal32_.get());
     }
 }
 
@@ -682,6 +688,7 @@ void DeviceBatch::setupMatrix(const double* diag, const double* upper, const dou
 template <class T>
 void DeviceBatch::recordSmooth(int k, const T* r, T* x, SmootherKind sm, bool pre, int flag, bool head) {
     DevLevel& D = L_[k];
+    constexpr int P = sizeof(T) == 4 ? 1 : 0;
     cudaStream_t s = stream_;
     const Sell S = D.sell();
     const T* val = LV<T>::val(D);
@@ -694,7 +701,7 @@ void DeviceBatch::recordSmooth(int k, const T* r, T* x, SmootherKind sm, bool pr
     if (jacobiHere) {
         // Jacobi; pre: from zero, post: after the ascent's prolongation pass
         const T om = T(jacobiOmega_);
-        const ChunkList& rows = head ? D.headActive : D.active;
+        const ChunkList& rows = head ? D.headActive[P] : D.active;
         if (pre && fusedLevel(k, fusePre_)) {
             // both sweeps from zero in one pass
             VLM_LAUNCH((k_smooth_jacobi<T, 3>), rows.n, kRowsPerCta, s, D.ch(rows), S, val, diag, r,
@@ -739,7 +746,7 @@ void DeviceBatch::recordSmooth(int k, const T* r, T* x, SmootherKind sm, bool pr
         // needed) and the post-smoothing's first colour applies the prolongation to the
         // neighbours it reads (no separate prolongation).
         const bool two = D.nSteps == 2;
-        const ChunkList& rows = head ? D.headActive : D.active;
+        const ChunkList& rows = head ? D.headActive[P] : D.active;
         if (pre && !two) VLM_LAUNCH(k_zero_rows<T>, rows.n, kRowsPerCta, s, D.ch(rows), x, st, flag);
         const bool boxK = k == 0 && boxOn_;
         const T* bc = LV<T>::bcoef(D);
@@ -761,15 +768,15 @@ void DeviceBatch::recordSmooth(int k, const T* r, T* x, SmootherKind sm, bool pr
                 VLM_CUDA(cudaEventRecord(te0, s));
             }
             if (boxK && two) {
-                const ChunkList& la = head ? (pre ? D.headFwd[0] : D.headRev[0]) : (pre ? D.fwd[0] : D.rev[0]);
-                const ChunkList& lb = head ? (pre ? D.headFwd[1] : D.headRev[1]) : (pre ? D.fwd[1] : D.rev[1]);
+                const ChunkList& la = head ? (pre ? D.headFwd[P][0] : D.headRev[P][0]) : (pre ? D.fwd[0] : D.rev[0]);
+                const ChunkList& lb = head ? (pre ? D.headFwd[P][1] : D.headRev[P][1]) : (pre ? D.fwd[1] : D.rev[1]);
                 if (recordFusedSweep<T>(la, lb, r, x, pre, sweep, agg, xc)) {
                     sweepEnd();
                     continue;
                 }
             }
             for (int t = 0; t < D.nSteps; ++t) {
-                const ChunkList& l = head ? (pre ? D.headFwd[t] : D.headRev[t]) : (pre ? D.fwd[t] : D.rev[t]);
+                const ChunkList& l = head ? (pre ? D.headFwd[P][t] : D.headRev[P][t]) : (pre ? D.fwd[t] : D.rev[t]);
                 if (boxK) {
                     int g = 0;
                     const BoxRows R = boxRows(D, l, &g);
@@ -896,17 +903,18 @@ template <class T>
 void DeviceBatch::recordVcycle(const T* r0, T* x0, SmootherKind sm, int flag, bool allowTail) {
     cudaStream_t s = stream_;
     const int nL = int(L_.size());
+    constexpr int P = sizeof(T) == 4 ? 1 : 0;
     const SysState* st = st_.get();
     auto rr = [&](int k) -> const T* { return k == 0 ? r0 : LV<T>::r(L_[k]); };
     auto xx = [&](int k) -> T* { return k == 0 ? x0 : LV<T>::x(L_[k]); };
     // Jacobi coarse levels: each system's levels from tailFirst_ down run in one cluster launch
     const bool tail = allowTail && tailOn_ && sm != SmootherKind::MCGS;
-    const int headEnd = tail ? tailMaxFirst_ : nL - 1;
+    const int headEnd = tail ? tailMaxFirst_[P] : nL - 1;
     for (int k = 0; k < headEnd; ++k) {
         DevLevel& D = L_[k];
         DevLevel& N = L_[k + 1];
-        const ChunkList& rows = tail ? D.headActive : D.active;
-        const ChunkList& next = tail ? N.headIn : N.all;
+        const ChunkList& rows = tail ? D.headActive[P] : D.active;
+        const ChunkList& next = tail ? N.headIn[P] : N.all;
         recordSmooth<T>(k, rr(k), xx(k), sm, true, flag, tail);
         if (k == 0 && boxOn_) {
             int g = 0;
@@ -946,7 +954,7 @@ void DeviceBatch::recordVcycle(const T* r0, T* x0, SmootherKind sm, int flag, bo
         // per k_prolong thread)
         const bool fusedProlong = jacobiHere && fusedLevel(k, fusePost_);
         if (!fusedProlong && (jacobiHere || (!D.blockGS && D.nSteps != 2))) {
-            const ChunkList& rows = tail ? D.headActive : D.active;
+            const ChunkList& rows = tail ? D.headActive[P] : D.active;
             VLM_LAUNCH(k_prolong<T>, rows.n, kRowsPerCta, s, D.ch(rows), D.agg.get(), xx(k + 1), xx(k), st, flag);
         }
         recordSmooth<T>(k, rr(k), xx(k), sm, false, flag, tail);
@@ -959,14 +967,23 @@ void DeviceBatch::recordTail(const T* r0, T* x0, int flag, bool jacobi0) {
                                                              : (const TailLevel<T>*)tail64_.get();
     if (!tab) throw Error(VLM_ERR_CUDA, "internal: coarse-tail table missing");
     if (tailSmem_) {
-        // every operand in shared memory, one CTA per system
+        // every operand in shared memory, one CTA or one cluster per system
+        constexpr bool f32 = std::is_same<T, float>::value;
+        const TailSmem& Q = tailPart_[f32 ? 1 : 0];
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(unsigned(tailImg_.size()));
-        cfg.blockDim = dim3(unsigned(kTailThreads));
-        cfg.dynamicSmemBytes = std::is_same<T, float>::value ? tailSmem32_ : tailSmem64_;
+        cfg.gridDim = dim3(unsigned(Q.systems) * unsigned(Q.cluster));
+        cfg.blockDim = dim3(unsigned(kTailPartThreads));
+        cfg.dynamicSmemBytes = Q.bytes;
         cfg.stream = stream_;
-        cudaLaunchAttribute at[1];
+        cudaLaunchAttribute at[2];
         int na = 0;
+        if (Q.cluster > 1) {
+            at[na].id = cudaLaunchAttributeClusterDimension;
+            at[na].val.clusterDim.x = unsigned(Q.cluster);
+            at[na].val.clusterDim.y = 1;
+            at[na].val.clusterDim.z = 1;
+            ++na;
+        }
         if (pdlEnabled()) {
             at[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
             at[na].val.programmaticStreamSerializationAllowed = 1;
@@ -974,10 +991,18 @@ void DeviceBatch::recordTail(const T* r0, T* x0, int flag, bool jacobi0) {
         }
         cfg.attrs = at;
         cfg.numAttrs = unsigned(na);
-        const T* vimg = std::is_same<T, float>::value ? (const T*)tailVal32_.get() : (const T*)tailVal64_.get();
-        VLM_CUDA(cudaLaunchKernelEx(&cfg, k_vcycle_tail_smem<T>, (const TailImg*)tailImg_.get(), vimg,
-                                    (const uint16_t*)tailStr_.get(), tab, (const double*)inv_.get(), T(jacobiOmega_),
-                                    (const SysState*)st_.get(), flag));
+        const T* vimg = f32 ? (const T*)tailVal32_.get() : (const T*)tailVal64_.get();
+        auto launch = [&](auto kernel) {
+            VLM_CUDA(cudaLaunchKernelEx(&cfg, kernel, (const TailPart*)Q.parts.get(), vimg,
+                                        (const uint16_t*)Q.str.get(), tab, (const double*)inv_.get(), r0, x0,
+                                        T(jacobiOmega_), (const SysState*)st_.get(), flag, jacobi0 ? 1 : 0));
+        };
+        switch (Q.cluster) {
+        case 8: launch(k_vcycle_tail_parts<T, 8>); break;
+        case 4: launch(k_vcycle_tail_parts<T, 4>); break;
+        case 2: launch(k_vcycle_tail_parts<T, 2>); break;
+        default: launch(k_vcycle_tail_parts<T, 1>); break;
+        }
         ++tl_launches;
         return;
     }
@@ -1016,100 +1041,158 @@ void DeviceBatch::recordTail(const T* r0, T* x0, int flag, bool jacobi0) {
     ++tl_launches;
 }
 
-// Per system: the first level of the single-CTA tail = the first level (below level 0) whose
-// padded row count is at most kTailMaxRows (VLM_TAIL_ROWS overrides; VLM_TAIL=0 disables), else
-// the coarsest level alone.
+// Per system: the first level of the tail = the first level (below level 0) whose padded row count
+// is at most the row limit (VLM_TAIL_ROWS overrides; VLM_TAIL=0 disables), else the coarsest level
+// alone; the whole V-cycle for systems of at most the full-row limit.  Without a wider global-memory
+// cluster asked for, the tail runs in shared memory on one cluster per system, as wide as lets
+// every system's cluster be resident at once (tailClusterFor), and the limits scale with that width:
+// a level has at most one row per thread of the cluster.
 void DeviceBatch::planTail() {
     const char* tv = std::getenv("VLM_TAIL");
     if (tv && tv[0] == '0') return;
     const int ns = plan_.nsys;
     if (ns == 0) return;
-    // the tail runs on one CTA or on a cluster of tailCl_ CTAs; unset row limits (0) scale with it
     if (tailCl_ != 1 && tailCl_ != 2 && tailCl_ != 4 && tailCl_ != 8)
         throw Error(VLM_ERR_BAD_ARG, "the coarse-tail cluster size must be 1, 2, 4 or 8");
-    const int64_t maxRows = tailMaxRows_ > 0 ? tailMaxRows_ : int64_t(kTailMaxRows) * tailCl_;
-    const int64_t fullRows =
-        tailFullRows_ > 0 ? tailFullRows_ : (tailCl_ == 1 ? int64_t(kTailFullRows) : int64_t(kTailMaxRows) * tailCl_);
     const LevelPlan& L0 = plan_.levels[0];
-    tailFirst_.assign(size_t(ns), 0);
-    std::vector<TailSys> ts(static_cast<size_t>(ns));
-    tailMaxFirst_ = 0;
-    for (int b = 0; b < ns; ++b) {
-        const int c = plan_.nLevels[b] - 1;
-        if (c >= kTailMaxLevels) throw Error(VLM_ERR_UNSUPPORTED, "GAMG hierarchy deeper than the coarse tail supports");
-        int first = c;
-        const int64_t rows0 = plan_.levels[0].sysRow[b + 1] - plan_.levels[0].sysRow[b];
-        if (c > 0 && rows0 <= fullRows && !plan_.levels[0].blockGS)
-            first = 0;  // the whole V-cycle of a small system in one CTA
-        else
-            for (int k = 1; k < c; ++k)
-                if (int64_t(plan_.levels[k].sysRow[b + 1] - plan_.levels[k].sysRow[b]) <= maxRows) {
-                    first = k;
-                    break;
-                }
-        tailFirst_[b] = first;
-        tailMaxFirst_ = std::max(tailMaxFirst_, first);
-        TailSys& t = ts[b];
-        std::memset(&t, 0, sizeof t);
-        t.sys = b;
-        t.first = first;
-        t.coarsest = c;
-        const CoarsePlan& cp = plan_.coarse[b];
-        t.coarseN = cp.n;
-        t.invOffset = cp.invOffset;
-        for (int k = 0; k <= c; ++k) {
-            t.rowStart[k] = plan_.levels[k].sysRow[b];
-            t.rowCount[k] = plan_.levels[k].sysRow[b + 1] - plan_.levels[k].sysRow[b];
+    auto starts = [&](int cluster) {
+        const int64_t maxRows = tailMaxRows_ > 0 ? tailMaxRows_ : int64_t(kTailMaxRows) * cluster;
+        const int64_t fullRows =
+            tailFullRows_ > 0 ? tailFullRows_ : (cluster == 1 ? int64_t(kTailFullRows) : int64_t(kTailMaxRows) * cluster);
+        std::vector<TailSys> ts(static_cast<size_t>(ns));
+        for (int b = 0; b < ns; ++b) {
+            const int c = plan_.nLevels[b] - 1;
+            if (c >= kTailMaxLevels) throw Error(VLM_ERR_UNSUPPORTED, "GAMG hierarchy deeper than the coarse tail supports");
+            int first = c;
+            const int64_t rows0 = L0.sysRow[b + 1] - L0.sysRow[b];
+            if (c > 0 && rows0 <= fullRows && !L0.blockGS)
+                first = 0;  // the whole V-cycle of a small system in the tail
+            else
+                for (int k = 1; k < c; ++k)
+                    if (int64_t(plan_.levels[k].sysRow[b + 1] - plan_.levels[k].sysRow[b]) <= maxRows) {
+                        first = k;
+                        break;
+                    }
+            TailSys& t = ts[b];
+            std::memset(&t, 0, sizeof t);
+            t.sys = b;
+            t.coarsest = c;
+            const CoarsePlan& cp = plan_.coarse[b];
+            t.coarseN = cp.n;
+            t.invOffset = cp.invOffset;
+            for (int k = 0; k <= c; ++k) {
+                t.rowStart[k] = plan_.levels[k].sysRow[b];
+                t.rowCount[k] = plan_.levels[k].sysRow[b + 1] - plan_.levels[k].sysRow[b];
+            }
+            // level-0 colour groups of this system (the chunks of the colour steps)
+            t.two = L0.nSteps == 2 ? 1 : 0;
+            t.nColours = 0;
+            for (int q = 0; q < L0.nSteps && q < 4; ++q) {
+                int s0 = -1, cnt = 0;
+                for (const Chunk& ch : L0.fwd[q])
+                    if (ch.sys == b) {
+                        if (s0 < 0) s0 = ch.start;
+                        cnt += ch.count;
+                    }
+                if (s0 < 0) break;
+                t.grpStart[q] = s0;
+                t.grpCount[q] = cnt;
+                t.nColours = q + 1;
+            }
+            if (first == 0 && L0.nSteps > 4) first = c;  // (never: level 0 is block-hybrid beyond 4 colours)
+            t.first = first;
+            if (cp.rowStart != t.rowStart[c]) throw Error(VLM_ERR_CUDA, "internal: coarse-tail row mismatch");
         }
-        // level-0 colour groups of this system (the chunks of the colour steps)
-        t.two = L0.nSteps == 2 ? 1 : 0;
-        t.nColours = 0;
-        for (int q = 0; q < L0.nSteps && q < 4; ++q) {
-            int s0 = -1, cnt = 0;
-            for (const Chunk& ch : L0.fwd[q])
-                if (ch.sys == b) {
-                    if (s0 < 0) s0 = ch.start;
-                    cnt += ch.count;
-                }
-            if (s0 < 0) break;
-            t.grpStart[q] = s0;
-            t.grpCount[q] = cnt;
-            t.nColours = q + 1;
-        }
-        if (first == 0 && L0.nSteps > 4) first = c;  // (never: level 0 is block-hybrid beyond 4 colours)
-        if (cp.rowStart != t.rowStart[c]) throw Error(VLM_ERR_CUDA, "internal: coarse-tail row mismatch");
+        return ts;
+    };
+    tailSmem_ = false;
+    if (tailSmemAllowed_ && tailCl_ == 1) {
+        const int cluster = tailClusterFor(ns);
+        std::vector<TailSys> ts = starts(cluster);
+        tailSmem_ = planTailSmem<double>(ts, cluster) && planTailSmem<float>(ts, cluster);
     }
-    tailSys_.upload(ts, stream_);
+    if (!tailSmem_) {  // one CTA or a cluster of tailCl_ CTAs per system on global memory
+        std::vector<TailSys> ts = starts(tailCl_);
+        for (int p = 0; p < 2; ++p) {
+            tailFirst_[p].clear();
+            for (const TailSys& t : ts) tailFirst_[p].push_back(t.first);
+        }
+        tailSys_.upload(ts, stream_);
+        VLM_CUDA(cudaStreamSynchronize(stream_));  // ts is a local
+    }
+    for (int p = 0; p < 2; ++p)
+        tailMaxFirst_[p] = *std::max_element(tailFirst_[p].begin(), tailFirst_[p].end());
     tailOn_ = true;
-    planTailSmem(ts);
 }
 
-// Images of the shared-memory tail (buildTailImages): used when every tail system qualifies.
-void DeviceBatch::planTailSmem(const std::vector<TailSys>& ts) {
-    tailSmem_ = false;
-    if (!tailSmemAllowed_ || tailCl_ != 1) return;
+namespace {
+
+// Bytes of dynamic shared memory a CTA of k_vcycle_tail_parts may use (its static descriptor aside).
+int tailBudget() {
     int dev = 0, optin = 0;
     VLM_CUDA(cudaGetDevice(&dev));
     VLM_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    const int budget = optin - int(sizeof(TailImg)) - 256;  // the kernel's static descriptor copy
-    TailImages im;
-    if (!buildTailImages(plan_, ts, size_t(budget), im)) return;
-    tailImg_.upload(im.imgs, stream_);
-    tailCodes_.upload(im.codes, stream_);
-    tailStr_.upload(im.str, stream_);
-    tailVal64_.resize(im.codes.size());
-    tailVal32_.resize(im.codes.size());
-    tailSmem64_ = im.bytes64;
-    tailSmem32_ = im.bytes32;
-    // the opt-in limit is a per-function setting: raised once to what the kernels may use
-    static const bool raised = [budget] {
-        VLM_CUDA(cudaFuncSetAttribute(k_vcycle_tail_smem<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, budget));
-        VLM_CUDA(cudaFuncSetAttribute(k_vcycle_tail_smem<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, budget));
-        return true;
+    return optin - int(sizeof(TailPart)) - 256;
+}
+
+// The opt-in limit is a per-function setting, raised once to what the kernels may use; returns how
+// many clusters of CL such CTAs the device holds at once.
+template <int CL>
+int tailClusters() {
+    static const int n = [] {
+        const int budget = tailBudget();
+        VLM_CUDA(cudaFuncSetAttribute(k_vcycle_tail_parts<double, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, budget));
+        VLM_CUDA(cudaFuncSetAttribute(k_vcycle_tail_parts<float, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, budget));
+        if (CL == 1) return 1 << 30;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(unsigned(CL));
+        cfg.blockDim = dim3(unsigned(kTailPartThreads));
+        cfg.dynamicSmemBytes = size_t(budget);
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = unsigned(CL);
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        int count = 0;
+        VLM_CUDA(cudaOccupancyMaxActiveClusters(&count, k_vcycle_tail_parts<double, CL>, &cfg));
+        return count;
     }();
-    (void)raised;
+    return n;
+}
+
+}  // namespace
+
+int DeviceBatch::tailClusterFor(int systems) {
+    if (systems <= tailClusters<8>()) return 8;
+    if (systems <= tailClusters<4>()) return 4;
+    if (systems <= tailClusters<2>()) return 2;
+    tailClusters<1>();
+    return 1;
+}
+
+// Images of the shared-memory tail in one precision (buildTailImages); false when a system's
+// coarsest level alone does not fit.
+template <class T>
+bool DeviceBatch::planTailSmem(std::vector<TailSys>& ts, int cluster) {
+    constexpr bool f32 = std::is_same<T, float>::value;
+    TailImages im;
+    if (!buildTailImages(plan_, ts, cluster, sizeof(T), size_t(tailBudget()), im)) return false;
+    TailSmem& Q = tailPart_[f32 ? 1 : 0];
+    Q.cluster = cluster;
+    Q.systems = int(ts.size());
+    Q.bytes = im.bytes;
+    Q.parts.upload(im.parts, stream_);
+    Q.codes.upload(im.codes, stream_);
+    Q.str.upload(im.str, stream_);
+    if (f32)
+        tailVal32_.resize(im.codes.size());
+    else
+        tailVal64_.resize(im.codes.size());
+    tailFirst_[f32 ? 1 : 0] = im.first;
     VLM_CUDA(cudaStreamSynchronize(stream_));  // the host vectors are locals
-    tailSmem_ = true;
+    return true;
 }
 
 void DeviceBatch::recordPrecond(PrecondKind pk, SmootherKind sm, const double* r, double* w, bool f32) {

@@ -26,8 +26,10 @@ struct DevLevel {
     DBuf<Chunk> chunks;
     std::vector<Chunk> hostChunks;  // host copy of `chunks`
     ChunkList active, all;
-    ChunkList headActive, headIn;  // coarse-tail mode: rows above each system's tail / restricted into
-    std::vector<ChunkList> headFwd, headRev;  // coarse-tail mode: colour steps of the systems above the tail
+    // coarse-tail mode, per precision (0: FP64, 1: FP32): rows above each system's tail / restricted
+    // into, and the colour steps of the systems above the tail
+    ChunkList headActive[2], headIn[2];
+    std::vector<ChunkList> headFwd[2], headRev[2];
     std::vector<ChunkList> fwd, rev;
     DBuf<int32_t> agg, childPtr, child, intraPtr, intraFace, cfacePtr, cfaceSrc;
     ChunkList coarse;  // CoarseDev entries whose coarsest level is this one
@@ -268,19 +270,24 @@ private:
     double jacobiOmega_ = 1.0;
     // coarse tail: levels tailFirst_[b].. of system b run in one CTA (Jacobi coarse levels)
     bool tailOn_ = false;
-    int tailMaxFirst_ = 0;      // head levels: k < tailMaxFirst_
-    std::vector<int> tailFirst_;
+    // per precision (0: FP64, 1: FP32): each system's first tail level; head levels: k < tailMaxFirst_
+    int tailMaxFirst_[2] = {0, 0};
+    std::vector<int> tailFirst_[2];
     DBuf<TailSys> tailSys_;
-    // shared-memory tail (k_vcycle_tail_smem): used when every tail system's levels fit
+    // shared-memory tail (k_vcycle_tail_parts): used when every system's coarsest levels fit
     bool tailSmem_ = false, tailSmemAllowed_ = true;
-    DBuf<TailImg> tailImg_;
-    DBuf<int32_t> tailCodes_;            // value-image gather codes (k_tail_values)
-    DBuf<uint16_t> tailStr_;             // structure images
+    struct TailSmem {
+        int cluster = 1, systems = 0;
+        size_t bytes = 0;                // dynamic shared memory per CTA
+        DBuf<TailPart> parts;
+        DBuf<int32_t> codes;             // value-image gather codes (k_tail_values)
+        DBuf<uint16_t> str;              // structure images
+    } tailPart_[2];
     DBuf<double> tailVal64_;
     DBuf<float> tailVal32_;
-    size_t tailSmem64_ = 0, tailSmem32_ = 0;  // dynamic shared memory per CTA
-    void planTailSmem(const std::vector<TailSys>& ts);
-    int tailCl_ = 1;                     // CTAs of the cluster that runs one system's tail (the tuner may widen it)
+    template <class T> bool planTailSmem(std::vector<TailSys>& ts, int cluster);
+    int tailClusterFor(int systems);
+    int tailCl_ = 1;                     // > 1: CTAs of the global-memory tail's cluster (asked for by setTail)
     int64_t tailMaxRows_ = 0;            // levels of at most this many rows go to the tail (0: scaled default)
     int64_t tailFullRows_ = 0;           // systems of at most this many level-0 rows: whole V-cycle there
     // fused coarse-level launches on levels of at most this many rows (all systems): both Jacobi

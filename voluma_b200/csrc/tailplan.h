@@ -1,4 +1,4 @@
-// Host-side construction of the shared-memory coarse tail's images (k_vcycle_tail_smem).
+// Host-side construction of the coarse tail's shared-memory images (k_vcycle_tail_parts).
 #pragma once
 
 #include <cstdint>
@@ -10,15 +10,17 @@
 namespace vlm {
 
 struct TailImages {
-    std::vector<TailImg> imgs;       // per tail system
+    std::vector<TailPart> parts;     // `cluster` consecutive parts per system
     std::vector<int32_t> codes;      // value-image gather codes (k_tail_values)
     std::vector<uint16_t> str;       // structure images
-    size_t bytes64 = 0, bytes32 = 0; // dynamic shared memory of the largest system, FP64 / FP32
+    std::vector<int> first;          // per system: the level its tail starts at
+    size_t bytes = 0;                // dynamic shared memory of the largest part
 };
 
-// Builds the images of every system of `ts` (levels first..coarsest): false when a system starts at
-// level 0, a level exceeds the 16-bit local indices, or a system's FP64 images and vectors exceed
-// `budget` bytes of shared memory.
-bool buildTailImages(const BatchPlan& plan, const std::vector<TailSys>& ts, size_t budget, TailImages& out);
+// Deals every system of `ts` to `cluster` CTAs: each system's tail starts at the first level from
+// ts[b].first on whose parts (values of `tsize` bytes) fit `budget` bytes of shared memory a CTA and
+// 16-bit local indices.  False when a system's coarsest level alone does not.
+bool buildTailImages(const BatchPlan& plan, const std::vector<TailSys>& ts, int cluster, size_t tsize, size_t budget,
+                     TailImages& out);
 
 }  // namespace vlm

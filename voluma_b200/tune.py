@@ -68,7 +68,8 @@ def apply(mesh) -> dict | None:
     e = lookup(entries, int(mesh.n_cells), int(getattr(mesh, "n_systems", 1)))
     if e is None:
         return None
-    mesh.set_tail(e["cluster"], e["max_rows"], e["full_rows"])
+    if (e["cluster"], e["max_rows"], e["full_rows"]) != mesh.tail_config():  # setting it re-plans the launches
+        mesh.set_tail(e["cluster"], e["max_rows"], e["full_rows"])
     return e
 
 
