@@ -288,6 +288,19 @@ def test_singular_coarsest_matrix_raises():
     assert e.value.name == "SINGULAR"
 
 
+@pytest.mark.parametrize("shape", [(2, 1, 1), (3, 3, 1), (4, 4, 2), (11, 3, 1), (7, 3, 3), (4, 4, 4), (9, 9, 9)])
+def test_coarse_factor_sizes(shape):
+    """The dense coarsest solve alone (systems of at most 64 cells have one level) at the edges of the
+    factor's row and column tiles, and under a hierarchy.  Bound: the inverse's rounding, both sides
+    substituting unit vectors through the same LU."""
+    M = vm.box_mesh(shape)
+    d, up = vm.poisson_matrix(M)
+    d = d - 0.1 * np.arange(1, M["n_cells"] + 1) / M["n_cells"]  # away from singular
+    r = np.random.default_rng(6).standard_normal(M["n_cells"])
+    w = vb.gamg_apply(vb.Mesh.from_arrays(M), d, up, None, r)
+    assert rel(w, ro.gamg_apply(M, d, up, None, r, smoother="mcgs-jacobi", coarse=1)) <= 1e-13
+
+
 def test_64cubed_gamg_against_oracle():
     M = vm.box_mesh((64, 64, 64), hi=(2 * np.pi,) * 3, periodic=(1, 1, 1))
     d, up = vm.poisson_matrix(M)

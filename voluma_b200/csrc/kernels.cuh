@@ -740,31 +740,161 @@ __global__ void __launch_bounds__(kRowsPerCta) k_prolong(const Chunk* __restrict
 
 // ------------------------------------------------------------------ coarsest level
 
-// Dense coarsest matrix, un-pivoted LU in place (GAMG.cpp:317-343) and the explicit
-// inverse from the LU by substituting unit vectors (GAMG.cpp:413-418 per column).
-// One CTA per system.  The factorisation runs in shared memory when the matrix fits
-// (smemN >= n: 2 n^2 doubles of dynamic shared memory), else in the global scratch `lu`.
-__global__ void k_coarse_factor(const CoarseDev* __restrict__ cs, Sell S, const double* __restrict__ val,
-                                const double* __restrict__ diag, double* __restrict__ lu, double* __restrict__ inv,
-                                int* status, int smemN) {
+// Dense coarsest matrix, un-pivoted LU (GAMG.cpp:317-343) and the explicit inverse from the LU by
+// substituting unit vectors (GAMG.cpp:413-418 per column), one CTA per system, n <= kCoarseSharedN.
+// A chain of 3 n dependent steps on one SM: what counts is the latency of a step.  The elements stay
+// in registers through the LU (thread (ty, tx): rows ty + 16 r, columns tx + 32 c), a step passes its
+// pivot row and column through shared memory and has one barrier; the columns of the inverse are
+// independent, so eight lanes carry one through both substitutions with shuffles and no barrier.
+// Every element sees the operations of the element-wise loops in their order (the same bits).
+// (A 64^2 cavity's ten SIMPLE steps 9.06 -> 8.84 ms against elements in shared memory and two
+// barriers a step.  With the substitutions' step loops rolled, less code to fetch, it measured 9.01.)
+constexpr int kCoarseSharedN = 80;  // larger coarsest matrices: k_coarse_factor_large
+constexpr int kCoarseThreads = 512;
+
+// Row i of the dense matrix: the diagonal, then the SELL entries in order (batched loads: the adds
+// may meet the same element twice).
+__device__ __forceinline__ void coarse_row(const Sell& S, const double* __restrict__ val,
+                                           const double* __restrict__ diag, int rowStart, int i, double* A) {
+    const int row = rowStart + i;
+    const int len = __ldg(S.rlen + row), base = sell_base(S, row);
+    A[i] = __ldg(diag + row);
+    for (int k0 = 0; k0 < len; k0 += kRowBatch) {
+        int j[kRowBatch];
+        double v[kRowBatch];
+#pragma unroll
+        for (int q = 0; q < kRowBatch; ++q)
+            if (k0 + q < len) {
+                const int e = base + ((k0 + q) << 5);
+                j[q] = __ldg(S.col + e) - rowStart;
+                v[q] = __ldg(val + e);
+            }
+#pragma unroll
+        for (int q = 0; q < kRowBatch; ++q)
+            if (k0 + q < len) A[j[q]] += v[q];
+    }
+}
+
+__global__ void __launch_bounds__(kCoarseThreads) k_coarse_factor(const CoarseDev* __restrict__ cs, Sell S,
+                                                                  const double* val, const double* diag, double* inv,
+                                                                  int* status) {
     pdl_entry();
-    extern __shared__ double sh[];
+    constexpr int NR = kCoarseSharedN / 16, NC = (kCoarseSharedN + 31) / 32, NX = kCoarseSharedN / 8;
+    extern __shared__ double A[];  // n rows of ld: an odd stride keeps column reads off one bank
+    __shared__ double rowb[2][kCoarseSharedN], colb[2][kCoarseSharedN];
+    const CoarseDev c = cs[blockIdx.x];
+    const int n = c.n, ld = n | 1;
+    const int tx = int(threadIdx.x) & 31, ty = int(threadIdx.x) >> 5;
+    for (int q = threadIdx.x; q < n * ld; q += kCoarseThreads) A[q] = 0.0;
+    __syncthreads();
+    if ((int)threadIdx.x < n) coarse_row(S, val, diag, c.rowStart, threadIdx.x, A + threadIdx.x * ld);
+    __syncthreads();
+    double a[NR][NC];
+#pragma unroll
+    for (int r = 0; r < NR; ++r)
+#pragma unroll
+        for (int q = 0; q < NC; ++q) {
+            const int i = ty + 16 * r, j = tx + 32 * q;
+            a[r][q] = i < n && j < n ? A[i * ld + j] : 0.0;
+        }
+    // row k and column k of the current block, for step k
+    auto publish = [&](int k) {
+        const int b = k & 1;
+#pragma unroll
+        for (int r = 0; r < NR; ++r)
+#pragma unroll
+            for (int q = 0; q < NC; ++q) {
+                const int i = ty + 16 * r, j = tx + 32 * q;
+                if (i == k && j < n) rowb[b][j] = a[r][q];
+                if (j == k && i < n) colb[b][i] = a[r][q];
+            }
+    };
+    publish(0);
+    __syncthreads();
+    for (int k = 0; k < n; ++k) {
+        const int b = k & 1;
+        const double piv = rowb[b][k];
+        if (fabs(piv) < kVSMALL) {  // uniform: every thread reads the same pivot
+            if (threadIdx.x == 0) atomicExch(status, (int)VLM_ERR_SINGULAR);
+            return;
+        }
+        // the multipliers of this warp's rows, one per lane; L and U go to A
+        double m = 0.0;
+        const int im = ty + 16 * tx;
+        if (tx < NR && im > k && im < n) {
+            m = colb[b][im] / piv;
+            A[im * ld + k] = m;
+        }
+        if (ty == (k & 15))
+            for (int j = k + tx; j < n; j += 32) A[k * ld + j] = rowb[b][j];
+        double u[NC];
+#pragma unroll
+        for (int q = 0; q < NC; ++q) u[q] = tx + 32 * q < n ? rowb[b][tx + 32 * q] : 0.0;
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            const double fct = __shfl_sync(0xffffffffu, m, r);
+            if (fct == 0.0) continue;  // uniform over the warp; rows up to k have no multiplier
+#pragma unroll
+            for (int q = 0; q < NC; ++q)
+                if (tx + 32 * q > k) a[r][q] -= fct * u[q];
+        }
+        if (k + 1 < n) publish(k + 1);
+        __syncthreads();
+    }
+    // column j of the inverse: eight lanes, rows 8 t + g of lane g.  Forward (unit L) from the unit
+    // vector, then backward (U).
+    const int g = tx & 7;
+    for (int j0 = 0; j0 < n; j0 += kCoarseThreads / 8) {
+        const int j = j0 + int(threadIdx.x) / 8;
+        double x[NX];
+#pragma unroll
+        for (int t = 0; t < NX; ++t) x[t] = 8 * t + g == j ? 1.0 : 0.0;
+#pragma unroll
+        for (int t = 0; t < NX; ++t)
+#pragma unroll
+            for (int s = 0; s < 8; ++s) {
+                const int k = 8 * t + s;
+                if (k + 1 >= n) break;
+                const double xk = __shfl_sync(0xffffffffu, x[t], s, 8);
+#pragma unroll
+                for (int w = t; w < NX; ++w) {
+                    const int i = 8 * w + g;
+                    if (i > k && i < n && j <= k) x[w] -= A[i * ld + k] * xk;
+                }
+            }
+#pragma unroll
+        for (int t = NX - 1; t >= 0; --t)
+#pragma unroll
+            for (int s = 7; s >= 0; --s) {
+                const int k = 8 * t + s;
+                if (k >= n) continue;
+                if (g == s) x[t] /= A[k * ld + k];
+                const double xk = __shfl_sync(0xffffffffu, x[t], s, 8);
+#pragma unroll
+                for (int w = 0; w <= t; ++w) {
+                    const int i = 8 * w + g;
+                    if (i < k) x[w] -= A[i * ld + k] * xk;
+                }
+            }
+        if (j < n)
+#pragma unroll
+            for (int t = 0; t < NX; ++t)
+                if (8 * t + g < n) inv[c.invOffset + (8 * t + g) * n + j] = x[t];
+    }
+}
+
+// The same for coarsest matrices beyond kCoarseSharedN rows, element by element in the global scratch.
+__global__ void k_coarse_factor_large(const CoarseDev* __restrict__ cs, Sell S, const double* __restrict__ val,
+                                      const double* __restrict__ diag, double* __restrict__ lu,
+                                      double* __restrict__ inv, int* status) {
+    pdl_entry();
     const CoarseDev c = cs[blockIdx.x];
     const int n = c.n;
-    const bool inShared = n <= smemN;
-    double* A = inShared ? sh : lu + c.invOffset;
-    double* X = inShared ? sh + (size_t)n * n : inv + c.invOffset;
+    double* A = lu + c.invOffset;
+    double* X = inv + c.invOffset;
     for (int q = threadIdx.x; q < n * n; q += blockDim.x) A[q] = 0.0;
     __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const int row = c.rowStart + i;
-        A[(size_t)i * n + i] = diag[row];
-        const int len = S.rlen[row], base = sell_base(S, row);
-        for (int k = 0; k < len; ++k) {
-            const int e = base + (k << 5);
-            A[(size_t)i * n + (S.col[e] - c.rowStart)] += val[e];
-        }
-    }
+    for (int i = threadIdx.x; i < n; i += blockDim.x) coarse_row(S, val, diag, c.rowStart, i, A + (size_t)i * n);
     __syncthreads();
     // LU without pivoting, one pivot at a time: multipliers of column k, then the trailing block
     // element-parallel (each element receives its updates in the order k = 0, 1, ...).  The block
@@ -808,9 +938,6 @@ __global__ void k_coarse_factor(const CoarseDev* __restrict__ cs, Sell S, const 
             for (int j = tx; j < n; j += 32) X[(size_t)i * n + j] -= u * X[(size_t)k * n + j];
         }
         __syncthreads();
-    }
-    if (inShared) {
-        for (int q = threadIdx.x; q < n * n; q += blockDim.x) inv[c.invOffset + q] = X[q];
     }
 }
 

@@ -94,9 +94,6 @@ namespace {
 
 inline int nblk(int n, int t = 256) { return (n + t - 1) / t; }
 
-// Coarsest matrices up to this order are factorised in shared memory (2 n^2 doubles).
-constexpr int kCoarseSharedN = 80;
-
 // Kernels enqueued (or captured) by this thread; solve() turns captured counts into executed ones.
 thread_local int64_t tl_launches = 0;
 
@@ -659,19 +656,21 @@ void DeviceBatch::setupMatrix(const double* diag, const double* upper, const dou
         int nmax = 0;
         for (const auto& c : plan_.coarse)
             if (c.level == k) nmax = std::max(nmax, c.n);
-        const int smemN = nmax <= kCoarseSharedN ? nmax : 0;
-        const size_t smem = size_t(2) * smemN * smemN * sizeof(double);
-        // the opt-in limit is per function and shared by every mesh: raised once to the ceiling
-        static const bool raised = [] {
-            VLM_CUDA(cudaFuncSetAttribute(k_coarse_factor, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          int(size_t(2) * kCoarseSharedN * kCoarseSharedN * sizeof(double))));
-            return true;
-        }();
-        (void)raised;
-        k_coarse_factor<<<D.coarse.n, 512, smem, s>>>(coarse_.get() + D.coarse.off, D.sell(), D.val.get(),
-                                                     D.diag.get(), lu_.get(), inv_.get(), status_.get(), smemN);
-        VLM_CUDA(cudaGetLastError());
-        ++tl_launches;
+        const CoarseDev* cs = coarse_.get() + D.coarse.off;
+        if (nmax <= kCoarseSharedN) {
+            // the opt-in limit is per function and shared by every mesh: raised once to the ceiling
+            static const bool raised = [] {
+                VLM_CUDA(cudaFuncSetAttribute(k_coarse_factor, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              int(size_t(kCoarseSharedN) * (kCoarseSharedN | 1) * sizeof(double))));
+                return true;
+            }();
+            (void)raised;
+            VLM_LAUNCH_SMEM(k_coarse_factor, D.coarse.n, kCoarseThreads, size_t(nmax) * size_t(nmax | 1) * sizeof(double),
+                            s, cs, D.sell(), (const double*)D.val.get(), (const double*)D.diag.get(), inv_.get(),
+                            status_.get());
+        } else
+            VLM_LAUNCH(k_coarse_factor_large, D.coarse.n, kCoarseThreads, s, cs, D.sell(), (const double*)D.val.get(),
+                       (const double*)D.diag.get(), lu_.get(), inv_.get(), status_.get());
     }
     if (tailOn_ && tailSmem_) {
         // the shared-memory tail's value images of this solve's coarse levels
