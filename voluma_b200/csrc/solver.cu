@@ -685,7 +685,7 @@ void DeviceBatch::setupMatrix(const double* diag, const double* upper, const dou
 
 // ====================================================================== V-cycle
 template <class T>
-void DeviceBatch::recordSmooth(int k, const T* r, T* x, SmootherKind sm, bool pre, int flag, bool head) {
+void DeviceBatch::recordSmooth(int k, const T* r, T* x, SmootherKind sm, bool pre, int flag, bool head, bool swept) {
     DevLevel& D = L_[k];
     constexpr int P = sizeof(T) == 4 ? 1 : 0;
     cudaStream_t s = stream_;
@@ -712,8 +712,9 @@ void DeviceBatch::recordSmooth(int k, const T* r, T* x, SmootherKind sm, bool pr
             VLM_LAUNCH((k_smooth_jacobi<T, 0>), rows.n, kRowsPerCta, s, D.ch(rows), S, val, diag, r, x2, x,
                        om, agg, xc, st, flag);
         } else if (pre) {
-            VLM_LAUNCH((k_smooth_jacobi<T, 1>), rows.n, kRowsPerCta, s, D.ch(rows), S, val, diag, r,
-                       (const T*)nullptr, x2, om, agg, xc, st, flag);
+            if (!swept)  // the restriction into this level has done the first sweep
+                VLM_LAUNCH((k_smooth_jacobi<T, 1>), rows.n, kRowsPerCta, s, D.ch(rows), S, val, diag, r,
+                           (const T*)nullptr, x2, om, agg, xc, st, flag);
             VLM_LAUNCH((k_smooth_jacobi<T, 0>), rows.n, kRowsPerCta, s, D.ch(rows), S, val, diag, r, x2, x,
                        om, agg, xc, st, flag);
         } else {
@@ -909,12 +910,14 @@ void DeviceBatch::recordVcycle(const T* r0, T* x0, SmootherKind sm, int flag, bo
     // Jacobi coarse levels: each system's levels from tailFirst_ down run in one cluster launch
     const bool tail = allowTail && tailOn_ && sm != SmootherKind::MCGS;
     const int headEnd = tail ? tailMaxFirst_[P] : nL - 1;
+    bool swept = false;  // level k's first Jacobi sweep is in its x2 already
     for (int k = 0; k < headEnd; ++k) {
         DevLevel& D = L_[k];
         DevLevel& N = L_[k + 1];
         const ChunkList& rows = tail ? D.headActive[P] : D.active;
         const ChunkList& next = tail ? N.headIn[P] : N.all;
-        recordSmooth<T>(k, rr(k), xx(k), sm, true, flag, tail);
+        recordSmooth<T>(k, rr(k), xx(k), sm, true, flag, tail, swept);
+        swept = false;
         if (k == 0 && boxOn_) {
             int g = 0;
             const BoxRows R = boxRows(D, rows, &g);
@@ -932,8 +935,11 @@ void DeviceBatch::recordVcycle(const T* r0, T* x0, SmootherKind sm, int flag, bo
         } else
             VLM_LAUNCH(k_residual<T>, rows.n, kRowsPerCta, s, D.ch(rows), D.sell(), LV<T>::val(D), LV<T>::diag(D),
                        rr(k), xx(k), LV<T>::t(D), st, flag);
+        // level k + 1 smooths by per-level Jacobi launches: its first sweep goes with the restriction
+        // (systems whose tail starts there ignore what this writes)
+        swept = k + 1 < headEnd && sm != SmootherKind::MCGS && !fusedLevel(k + 1, fusePre_);
         VLM_LAUNCH(k_restrict<T>, next.n, kRowsPerCta, s, N.ch(next), D.childPtr.get(), D.child.get(), LV<T>::t(D),
-                   LV<T>::r(N), st, flag);
+                   LV<T>::r(N), LV<T>::diag(N), T(jacobiOmega_), swept ? LV<T>::x2(N) : (T*)nullptr, st, flag);
     }
     if (tail) {
         recordTail<T>(r0, x0, flag, sm == SmootherKind::Jacobi);
@@ -956,7 +962,7 @@ void DeviceBatch::recordVcycle(const T* r0, T* x0, SmootherKind sm, int flag, bo
             const ChunkList& rows = tail ? D.headActive[P] : D.active;
             VLM_LAUNCH(k_prolong<T>, rows.n, kRowsPerCta, s, D.ch(rows), D.agg.get(), xx(k + 1), xx(k), st, flag);
         }
-        recordSmooth<T>(k, rr(k), xx(k), sm, false, flag, tail);
+        recordSmooth<T>(k, rr(k), xx(k), sm, false, flag, tail, false);
     }
 }
 

@@ -216,7 +216,8 @@ private:
 
 private:
     template <class T> void recordVcycle(const T* r0, T* x0, SmootherKind sm, int flag, bool allowTail = true);
-    template <class T> void recordSmooth(int k, const T* r, T* x, SmootherKind sm, bool pre, int flag, bool head);
+    template <class T> void recordSmooth(int k, const T* r, T* x, SmootherKind sm, bool pre, int flag, bool head,
+                                         bool swept);
     template <class T> void recordTail(const T* r0, T* x0, int flag, bool jacobi0);
     template <class T> void buildTailTable(DBuf<TailLevel<T>>& out);
     void planTail();
