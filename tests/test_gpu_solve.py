@@ -428,7 +428,7 @@ def test_shared_memory_tail_matches_global_tail(name, precision, monkeypatch):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("shape,periodic", [((5, 5, 5), (1, 1, 1)), ((9, 7, 5), (1, 0, 0)), ((20, 20, 20), (0, 0, 0)),
+@pytest.mark.parametrize("shape,periodic", [((5, 5, 5), (1, 1, 1)), ((9, 7, 5), (1, 0, 0)), ((8, 8, 8), (1, 1, 1)), ((20, 20, 20), (0, 0, 0)),
                                             ((64, 64, 1), (0, 0, 0)), ((32, 31, 19), (0, 1, 0))])
 @pytest.mark.parametrize("smoother", ["mcgs-jacobi", "jacobi"])
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])

@@ -1112,8 +1112,13 @@ void DeviceBatch::planTail() {
     };
     tailSmem_ = false;
     if (tailSmemAllowed_ && tailCl_ == 1) {
-        const int cluster = tailClusterFor(ns);
+        int cluster = tailClusterFor(ns);
         std::vector<TailSys> ts = starts(cluster);
+        // at most one row per thread of one CTA on every level: its own barrier is shorter than the
+        // cluster's (480 cells, 11 iterations: 0.65 -> 0.61 ms a solve).  Running only the levels below
+        // 512 rows of a larger tail that way measured slower (96^3 FP64 11.26 -> 11.39 ms).
+        if (std::all_of(ts.begin(), ts.end(), [](const TailSys& t) { return t.rowCount[t.first] <= kTailPartThreads; }))
+            cluster = tailClusterFor(1 << 30);
         tailSmem_ = planTailSmem<double>(ts, cluster) && planTailSmem<float>(ts, cluster);
     }
     if (!tailSmem_) {  // one CTA or a cluster of tailCl_ CTAs per system on global memory
