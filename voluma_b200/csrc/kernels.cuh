@@ -167,8 +167,8 @@ __device__ bool reduce_exact_bins(long long (*bins)[kRowsPerCta / 32][kExactBins
     if (!isLast) return false;
     __threadfence();
     // each warp adds every kWarps-th slot's words, four slots' loads in flight, into its own bins.
-    // With the windows above and the span of exact_value, a reduction kernel of the reproducible PCG at
-    // 43,200 rows (43 CTAs) takes 9 us instead of 31 (275 iterations: 26.6 -> 9.9 ms).
+    // A reduction kernel of the reproducible PCG took 31 us at 43,200 rows (43 CTAs); with the windows and
+    // the span of exact_value as well, 275 iterations of three such kernels went from 26.6 to 9.9 ms.
     constexpr int kWords = NV * kExactStride, kPer = (kWords + 31) / 32;
     __shared__ long long tot[NV][kExactStride];
     const int b0 = R.slotBegin[c.sys], b1 = R.slotEnd[c.sys];
