@@ -12,6 +12,8 @@ The level-scheduled kernels apply every row's terms in the reference's order, so
     in the true residual, and match its solution within 1e-10 (PCG/DIC) or 1e-6 (PBiCGStab/DILU,
     whose iterates amplify the reductions' rounding to the solver tolerance).
 """
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -157,6 +159,53 @@ def test_pipelined_parts_apply_bitwise(n, periodic, two_d):
         r = rng.standard_normal(msh["n_cells"])
         w = vb.precond_apply(m, diag, upper, lower, r, "DILU")
         assert np.array_equal(w, ro.precond_apply(msh, diag, upper, lower, r, "DILU"))
+
+
+class _filled_block:
+    """Device memory from the driver's allocator (the one behind the library's), every double 2.2e6."""
+
+    def __init__(self, nbytes):
+        self.cu = ctypes.CDLL("libcuda.so.1")
+        self.p = ctypes.c_uint64()
+        assert self.cu.cuMemAlloc_v2(ctypes.byref(self.p), ctypes.c_size_t(nbytes)) == 0
+        assert self.cu.cuMemsetD32_v2(self.p, ctypes.c_uint32(0x41412121), ctypes.c_size_t(nbytes // 4)) == 0
+
+    def free(self):
+        assert self.cu.cuMemFree_v2(self.p) == 0
+
+
+@pytest.mark.parametrize("n,periodic,two_d", [
+    ((41, 35, 29), (1, 0, 1), False),  # odd rows of a box: padding inside every row's colour group
+    ((97, 83, 1), (0, 0, 0), True),
+])
+def test_wide_solve_does_not_depend_on_what_its_memory_held(n, periodic, two_d):
+    """PBiCGStab reduces over padding rows too, so the sweeps have to leave them at zero: the solve
+    of a mesh whose vectors land in memory that held large values is the oracle's, at its first
+    call and after a call of another solver."""
+    from voluma_b200 import mesh as vm
+    msh = vm.box_mesh(n, hi=(1.0, 1.0, 1.0), periodic=periodic, two_d=two_d)
+    diag, upper = vm.poisson_matrix(msh)
+    diag = 1.05 * diag  # well conditioned: converged solutions agree however the sums were rounded
+    rng = np.random.default_rng(13)
+    lower = upper * (0.8 + 0.4 * rng.random(msh["n_internal_faces"]))
+    b = rng.standard_normal(msh["n_cells"])
+    ctrl = vb.SolverControls("PBiCGStab", "DILU", 0.0, 1e-10, 200)
+    xo, po = ro.solve(msh, diag, upper, lower, b, np.zeros(msh["n_cells"]), "PBiCGStab", "DILU", 0.0, 1e-10, 200)
+    # every other block of one vector's size keeps the allocator's pages, the rest goes back to it
+    m = vb.Mesh.from_arrays(msh)
+    blocks = [_filled_block(8 * (msh["n_cells"] + 2048)) for _ in range(256)]
+    for q in blocks[::2]:
+        q.free()
+    try:
+        for _ in range(2):
+            x = np.zeros(msh["n_cells"])
+            p = vb.solve_ldu(m, diag, upper, lower, b, x, ctrl)
+            assert abs(p.iterations - po["iterations"]) <= 1
+            assert rel(x, xo) <= 1e-8  # both stop at 1e-10 of the initial residual; condition below 100
+            vb.solve_ldu(m, diag, upper, lower, b, x, vb.SolverControls("PBiCGStab", "diagonal", 0.0, 1e-2, 20))
+    finally:
+        for q in blocks[1::2]:
+            q.free()
 
 
 def test_pipelined_parts_of_a_batch_match_solo():

@@ -132,10 +132,14 @@ DiluParts buildDiluParts(const DiluPlan& D, const BatchPlan& P, const std::vecto
         const int part0 = int(R.parts.size());
         std::vector<std::vector<int32_t>> rows(static_cast<size_t>(np));  // level by level
         std::vector<std::vector<int32_t>> ends(static_cast<size_t>(np));  // end of each non-empty level's rows
+        std::vector<int32_t> pads;
         for (int t = 0; t < ds.nLev; ++t) {
             for (int k = D.levPtr[ds.levBegin + t]; k < D.levPtr[ds.levBegin + t + 1]; ++k) {
                 const int r = D.levRows[k];
-                if (P.perm0[r] < 0) continue;  // padding: never written, no neighbours
+                if (P.perm0[r] < 0) {  // padding: no neighbours, no step
+                    pads.push_back(r);
+                    continue;
+                }
                 const int q = int((P.perm0[r] - cb) * np / n);
                 partOf[r] = part0 + q;
                 rows[q].push_back(r);
@@ -144,7 +148,11 @@ DiluParts buildDiluParts(const DiluPlan& D, const BatchPlan& P, const std::vecto
                 if (int(rows[q].size()) > (ends[q].empty() ? 0 : ends[q].back())) ends[q].push_back(int(rows[q].size()));
         }
         for (int q = 0; q < np; ++q) {
-            DiluPart part{ds.sys, int(R.steps.size()), 0, int(R.slotRow.size()), int(rows[q].size())};
+            DiluPart part{ds.sys, int(R.steps.size()), 0, int(R.slotRow.size()), int(rows[q].size()), 0, 0};
+            const size_t p0 = pads.size() * size_t(q) / size_t(np), p1 = pads.size() * size_t(q + 1) / size_t(np);
+            part.pad0 = int(R.padRow.size());
+            part.nPad = int(p1 - p0);
+            R.padRow.insert(R.padRow.end(), pads.begin() + std::ptrdiff_t(p0), pads.begin() + std::ptrdiff_t(p1));
             int a = 0;
             for (int e : ends[q])
                 while (a < e) {

@@ -62,9 +62,11 @@ DiluPlan buildDiluPlan(const std::vector<SysTopo>& systems, const BatchPlan& P);
 // part's forward sweep reads only its own rows and rows of earlier parts (its backward sweep, of
 // later parts): each part walks its own rows level by level and takes the values of other parts from
 // per-value mailboxes, so no two CTAs ever meet at a barrier.  Slots: every real row of a part, step by
-// step; a step is at most maxWidth rows of one level.
+// step; a step is at most maxWidth rows of one level.  A system's padding rows are dealt to its parts too:
+// the backward sweep leaves 0 there, which the reductions over all rows rely on.
 struct DiluPart {
     int sys, stepBegin, nSteps, slot0, nSlots;
+    int pad0, nPad;  // its padding rows in padRow
 };
 
 // Slots [s0, s0 + width); entry j of slot s0 + q at lo + j * width + q (up likewise): a slot of the part
@@ -77,6 +79,7 @@ struct DiluParts {
     std::vector<DiluPart> parts;  // forward order; the backward sweep takes them in reverse
     std::vector<DiluStep> steps;
     std::vector<int32_t> slotRow;                        // slot -> solver row
+    std::vector<int32_t> padRow;                         // padding rows, part by part
     std::vector<int32_t> loCol, loFace, upCol, upFace;   // entries (faces as DiluPlan's)
     std::vector<int32_t> loRemote, upRemote;             // mailbox of each remote entry
     std::vector<int32_t> loMail, upMail;                 // per slot: the mailbox its value goes to, -1: none

@@ -82,7 +82,7 @@ struct DiluPartArgs {
     const DiluStep* steps;
     int nParts, W, M, maxRemote;  // ring shape: slots, staged entries, remote entries per step
     int stepsLocal;               // the part's step descriptors are copied to shared memory
-    const int32_t* slotRow;
+    const int32_t *slotRow, *padRow;
     const int32_t *col, *remote, *mail;  // of the sweep's direction
     const double* coef;                  // per entry: A_lu A_ul (factor), A_ul (forward), A_lu (backward)
     DiluMail* box;                       // mailboxes of the direction
@@ -114,6 +114,8 @@ __global__ void __launch_bounds__(kPartThreads, 1) k_dilu_part(const DiluPartArg
     const DiluPart P = A.parts[sPart];
     const unsigned long long tag = sTag;
     if (A.st == nullptr || !sys_idle(A.st[P.sys], A.flag)) {  // uniform over the system's parts
+        if (KIND == kPartBackward)
+            for (int i = tid; i < P.nPad; i += kPartThreads) A.w[__ldg(A.padRow + P.pad0 + i)] = 0.0;
         double* sh = reinterpret_cast<double*>(psm);
         double* rem = reinterpret_cast<double*>(psm + dilu_align16(size_t(SH ? P.nSlots : 0) * sizeof(double)));
         const int W = A.W, M = A.M, maxRem = A.maxRemote;
@@ -277,7 +279,7 @@ struct DiluPipeArgs {
     const DiluPart* parts;
     const DiluRecStep* steps;
     int nParts, W, E, maxRemote, ring;  // ring shape: slots, extensions; stages
-    const int32_t* slotRow;
+    const int32_t *slotRow, *padRow;
     const int4* col;        // records of the sweep's direction
     const double* coef;     // four doubles per record: three coefficients, 1 / rD
     const int32_t* remote;  // mailbox of each remote entry
@@ -357,6 +359,8 @@ __global__ void __launch_bounds__(kPartThreads, 1) k_dilu_pipe(const DiluPipeArg
     const DiluPart P = A.parts[sPart];
     const unsigned long long tag = sTag;
     if (A.st == nullptr || !sys_idle(A.st[P.sys], A.flag)) {  // uniform over the system's parts
+        if (KIND == kPartBackward)
+            for (int i = tid; i < P.nPad; i += kPartThreads) A.w[__ldg(A.padRow + P.pad0 + i)] = 0.0;
         const int W = A.W, E = A.E, maxRem = A.maxRemote, nSteps = P.nSteps, R = A.ring;
         double* sh = reinterpret_cast<double*>(psm);
         double* rem = sh + P.nSlots;

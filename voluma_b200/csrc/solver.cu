@@ -42,7 +42,7 @@ struct DiluDev {
     // pipelined parts (dilupart.cuh): used otherwise; their entries are sLo* / sUp* above
     DBuf<DiluPart> parts;
     DBuf<DiluStep> steps;
-    DBuf<int32_t> loRemote, upRemote, loMail, upMail;
+    DBuf<int32_t> padRow, loRemote, upRemote, loMail, upMail;
     DBuf<DiluMail> loBox, upBox;
     DBuf<DiluPartSync> psync;
     DBuf<double> ws;
@@ -488,6 +488,8 @@ void DeviceBatch::ensureVectors(bool mixed, bool bicg) {
         s_.resize(n0);
         z_.resize(n0);
         t_.resize(n0);
+        // the padding rows of every vector stay 0 from here on: the reductions run over them
+        for (DBuf<double>* v : {&r0_, &y_, &Ay_, &s_, &z_, &t_}) v->zero(stream_);
     }
     if (mixed && e32_.size() != n0) {
         e32_.resize(n0);
@@ -1505,6 +1507,7 @@ void DeviceBatch::planDiluParts(DiluDev& D, const DiluPlan& P, int sms) {
     D.nParts = int(R.parts.size());
     D.parts.upload(R.parts, s);
     D.slotRow.upload(R.slotRow, s);
+    D.padRow.upload(R.padRow, s);
     D.loRemote.upload(R.loRemote, s);
     D.upRemote.upload(R.upRemote, s);
     D.loBox.resize(size_t(std::max(R.nLoMail, 1)));
@@ -1651,7 +1654,7 @@ void DeviceBatch::launchDiluPart(const double* src, double* w, const SysState* s
     constexpr bool back = KIND == kPartBackward;
     if (D.records) {
         const DiluPipeArgs A{D.parts.get(), D.recSteps.get(), D.nParts, D.W, D.maxExt, D.maxRemote, D.ring,
-                             D.slotRow.get(), (const int4*)(back ? D.recUpCol.get() : D.recLoCol.get()),
+                             D.slotRow.get(), D.padRow.get(), (const int4*)(back ? D.recUpCol.get() : D.recLoCol.get()),
                              KIND == kPartFactor ? D.prod.get() : back ? D.coefUp.get() : D.coefLo.get(),
                              back ? D.upRemote.get() : D.loRemote.get(), back ? D.upBox.get() : D.loBox.get(),
                              D.coefLo.get(), D.coefUp.get(), D.ws.get(), src, w, D.psync.get(), D.err.get(), st,
@@ -1660,7 +1663,7 @@ void DeviceBatch::launchDiluPart(const double* src, double* w, const SysState* s
         return;
     }
     const DiluPartArgs A{D.parts.get(), D.steps.get(), D.nParts, D.W, D.M, D.maxRemote, D.stepsLocal, D.slotRow.get(),
-                         back ? D.sUpCol.get() : D.sLoCol.get(), back ? D.upRemote.get() : D.loRemote.get(),
+                         D.padRow.get(), back ? D.sUpCol.get() : D.sLoCol.get(), back ? D.upRemote.get() : D.loRemote.get(),
                          back ? D.upMail.get() : D.loMail.get(),
                          KIND == kPartFactor ? D.prod.get() : back ? D.coefUp.get() : D.coefLo.get(),
                          back ? D.upBox.get() : D.loBox.get(), D.rDs.get(), D.ws.get(), src, w, D.psync.get(),
