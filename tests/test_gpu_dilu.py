@@ -263,3 +263,34 @@ def test_group_barrier_gives_up_when_a_cta_never_arrives():
     assert np.all(passed == 0)  # nobody got through the first barrier
     st, passed = vb.barrier_check(4, 1 << 22, absent_cta=-1, rounds=3)
     assert st == "OK" and np.all(passed == 3)
+
+
+@pytest.mark.parametrize("n", [(20000, 1, 1), (41, 35, 29)])
+def test_mailbox_wait_that_runs_out_ends_with_timeout(n, monkeypatch):
+    """A limit that a wait exceeds at once: the sweep still ends, with status TIMEOUT, and the next
+    application of the same mesh is right (general parts for the chain, records for the box)."""
+    from voluma_b200 import mesh as vm
+    msh = vm.box_mesh(n)
+    diag, upper = vm.poisson_matrix(msh)
+    r = np.random.default_rng(3).standard_normal(msh["n_cells"])
+    m = vb.Mesh.from_arrays(msh)
+    w = ro.precond_apply(msh, diag, upper, upper, r, "DILU")
+    for _ in range(2):
+        monkeypatch.setenv("VLM_MAIL_POLLS", "-1000000000")
+        with pytest.raises(vb.VlmError) as e:
+            vb.precond_apply(m, diag, upper, None, r, "DILU")
+        assert e.value.name == "TIMEOUT"
+        monkeypatch.delenv("VLM_MAIL_POLLS")
+        assert np.array_equal(vb.precond_apply(m, diag, upper, None, r, "DILU"), w)
+
+
+def test_mailbox_wait_grows_with_the_steps_before_it(monkeypatch):
+    """A chain of one row a level: its second part waits for all 10,000 steps of the first, ten times
+    as long as the polls that a wait has for itself."""
+    from voluma_b200 import mesh as vm
+    msh = vm.box_mesh((20000, 1, 1))
+    diag, upper = vm.poisson_matrix(msh)
+    r = np.random.default_rng(3).standard_normal(msh["n_cells"])
+    monkeypatch.setenv("VLM_MAIL_POLLS", "1000")
+    w = vb.precond_apply(vb.Mesh.from_arrays(msh), diag, upper, None, r, "DILU")
+    assert np.array_equal(w, ro.precond_apply(msh, diag, upper, upper, r, "DILU"))

@@ -770,7 +770,7 @@ void pressureLoop(vlm_mesh* m, const double* gamma, const double* divPhi, double
     for (int no = 0; no <= nNonOrth; ++no) {
         if (hst[2 * no + 1] != 0) {
             m->batch->clearLevelError();
-            throw vlm::Error(VLM_ERR_TIMEOUT, "level-scheduled sweep: a group barrier wait gave up");
+            throw vlm::Error(VLM_ERR_TIMEOUT, "level-scheduled sweep: a bounded wait gave up");
         }
         if (hst[2 * no] == VLM_ERR_SINGULAR) throw vlm::Error(VLM_ERR_SINGULAR, "GAMG: singular coarsest matrix");
         const vlm_solver_ctrl& c = no == nNonOrth ? finalCtrl : ctrl;

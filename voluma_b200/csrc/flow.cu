@@ -1784,7 +1784,7 @@ vlm_step_info DeviceFlow::step(double dt) {
         if (status[2 * k + 1] != 0) {
             batch_.clearLevelError();
             if (uBatch_) uBatch_->clearLevelError();
-            throw Error(VLM_ERR_TIMEOUT, "level-scheduled sweep: a group barrier wait gave up");
+            throw Error(VLM_ERR_TIMEOUT, "level-scheduled sweep: a bounded wait gave up");
         }
         if (status[2 * k] == VLM_ERR_SINGULAR) throw Error(VLM_ERR_SINGULAR, "GAMG: singular coarsest matrix");
         info.iterations += st[k].iterations;

@@ -46,7 +46,7 @@ struct DiluDev {
     DBuf<DiluMail> loBox, upBox;
     DBuf<DiluPartSync> psync;
     DBuf<double> ws;
-    int nParts = 0, maxRemote = 0;
+    int nParts = 0, nSteps = 0, maxRemote = 0;
     bool local = false;  // each part's vector in shared memory
     size_t partSmem = 0;
     int stepsLocal = 0;
@@ -1505,6 +1505,7 @@ void DeviceBatch::planDiluParts(DiluDev& D, const DiluPlan& P, int sms) {
     D.M = M;
     D.maxRemote = R.maxRemote;
     D.nParts = int(R.parts.size());
+    D.nSteps = int(R.steps.size());
     D.parts.upload(R.parts, s);
     D.slotRow.upload(R.slotRow, s);
     D.padRow.upload(R.padRow, s);
@@ -1652,12 +1653,16 @@ template <int KIND>
 void DeviceBatch::launchDiluPart(const double* src, double* w, const SysState* st) {
     DiluDev& D = *dilu_;
     constexpr bool back = KIND == kPartBackward;
+    // VLM_MAIL_POLLS: another limit (negative: a wait that has to poll gives up at once)
+    const char* mp = std::getenv("VLM_MAIL_POLLS");
+    const int polls = mp ? std::atoi(mp) : kMailPolls;
     if (D.records) {
         const DiluPipeArgs A{D.parts.get(), D.recSteps.get(), D.nParts, D.W, D.maxExt, D.maxRemote, D.ring,
                              D.slotRow.get(), D.padRow.get(), (const int4*)(back ? D.recUpCol.get() : D.recLoCol.get()),
                              KIND == kPartFactor ? D.prod.get() : back ? D.coefUp.get() : D.coefLo.get(),
                              back ? D.upRemote.get() : D.loRemote.get(), back ? D.upBox.get() : D.loBox.get(),
-                             D.coefLo.get(), D.coefUp.get(), D.ws.get(), src, w, D.psync.get(), D.err.get(), st,
+                             D.coefLo.get(), D.coefUp.get(), D.ws.get(), src, w, D.psync.get(), D.nSteps, polls,
+                             D.err.get(), st,
                              int(kFlagDone)};
         VLM_LAUNCH_SMEM(k_dilu_pipe<KIND>, D.nParts, kPartThreads, D.partSmem, stream_, A);
         return;
@@ -1667,7 +1672,7 @@ void DeviceBatch::launchDiluPart(const double* src, double* w, const SysState* s
                          back ? D.upMail.get() : D.loMail.get(),
                          KIND == kPartFactor ? D.prod.get() : back ? D.coefUp.get() : D.coefLo.get(),
                          back ? D.upBox.get() : D.loBox.get(), D.rDs.get(), D.ws.get(), src, w, D.psync.get(),
-                         D.err.get(), st, int(kFlagDone)};
+                         D.nSteps, polls, D.err.get(), st, int(kFlagDone)};
     if (D.local)
         VLM_LAUNCH_SMEM((k_dilu_part<KIND, true>), D.nParts, kPartThreads, D.partSmem, stream_, A);
     else
@@ -1681,7 +1686,7 @@ void DeviceBatch::clearLevelError() {
     dilu_->bars.zero(stream_);
 }
 
-// A group barrier of a level-scheduled kernel that gave up leaves its status here.
+// A bounded wait of a level-scheduled kernel that gave up leaves its status here.
 void DeviceBatch::checkLevelError() {
     int e = 0;
     VLM_CUDA(cudaMemcpy(&e, dilu_->err.get(), sizeof(int), cudaMemcpyDeviceToHost));
@@ -1689,7 +1694,7 @@ void DeviceBatch::checkLevelError() {
         dilu_->err.zero(stream_);
         dilu_->bars.zero(stream_);
         VLM_CUDA(cudaStreamSynchronize(stream_));
-        throw Error(VLM_ERR_TIMEOUT, "level-scheduled sweep: a group barrier wait gave up");
+        throw Error(VLM_ERR_TIMEOUT, "level-scheduled sweep: a bounded wait gave up");
     }
 }
 
