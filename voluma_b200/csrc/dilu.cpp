@@ -121,6 +121,16 @@ DiluPlan buildDiluPlan(const std::vector<SysTopo>& systems, const BatchPlan& P) 
     return D;
 }
 
+int diluWidth(const DiluPlan& D, const DiluSys& ds, const BatchPlan& P) {
+    int width = 0;
+    for (int t = 0; t < ds.nLev; ++t) {
+        const auto a = D.levRows.begin() + D.levPtr[ds.levBegin + t], e = D.levRows.begin() + D.levPtr[ds.levBegin + t + 1];
+        const auto real = t == 0 ? std::count_if(a, e, [&](int r) { return P.perm0[r] >= 0; }) : e - a;
+        width = std::max(width, int(real));
+    }
+    return width;
+}
+
 DiluParts buildDiluParts(const DiluPlan& D, const BatchPlan& P, const std::vector<int>& nParts, int maxWidth) {
     DiluParts R;
     const int nrows = int(P.perm0.size());

@@ -54,6 +54,9 @@ struct DiluPlan {
     int maxRows = 0;   // largest system (level-0 rows incl. padding)
 };
 
+// Rows of a system's widest level, its padding rows (which sit on level 0 and are in no step) left out.
+int diluWidth(const DiluPlan& D, const DiluSys& ds, const BatchPlan& P);
+
 // systems: input order; P: the batch plan (solver order, perm0).
 DiluPlan buildDiluPlan(const std::vector<SysTopo>& systems, const BatchPlan& P);
 

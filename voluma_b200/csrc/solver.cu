@@ -1438,11 +1438,9 @@ void DeviceBatch::planDiluParts(DiluDev& D, const DiluPlan& P, int sms) {
         std::vector<int> np(P.sys.size(), 1);
         int64_t total = 0;
         for (size_t b = 0; b < P.sys.size(); ++b) {
-            const DiluSys& ds = P.sys[b];
-            int width = 0;
-            for (int t = 0; t < ds.nLev; ++t)
-                width = std::max(width, P.levPtr[ds.levBegin + t + 1] - P.levPtr[ds.levBegin + t]);
-            if (!one) np[b] = std::max((width + kPartWidth - 1) / kPartWidth, maxSlots ? (ds.rowCount + maxSlots - 1) / maxSlots : 1);
+            const int width = diluWidth(P, P.sys[b], plan_), cells = plan_.sysCells[P.sys[b].sys];
+            if (!one)
+                np[b] = std::max({1, (width + kPartWidth - 1) / kPartWidth, maxSlots ? (cells + maxSlots - 1) / maxSlots : 1});
             total += np[b];
         }
         if (maxSlots && P.sys.size() == 1 && total > sms) return false;
