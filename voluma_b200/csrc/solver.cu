@@ -1651,16 +1651,16 @@ template <int KIND>
 void DeviceBatch::launchDiluPart(const double* src, double* w, const SysState* st) {
     DiluDev& D = *dilu_;
     constexpr bool back = KIND == kPartBackward;
-    // VLM_MAIL_POLLS: another limit (negative: a wait that has to poll gives up at once)
+    // VLM_MAIL_POLLS: another limit (negative: a wait gives up at its 64th poll)
     const char* mp = std::getenv("VLM_MAIL_POLLS");
-    const int polls = mp ? std::atoi(mp) : kMailPolls;
+    const int64_t polls = (mp ? std::atoll(mp) : kMailPolls) + int64_t(kMailStepPolls) * D.nSteps;
+    const int limit = int(std::max<int64_t>(-1, std::min<int64_t>(polls, 0x7fffff00)));
     if (D.records) {
         const DiluPipeArgs A{D.parts.get(), D.recSteps.get(), D.nParts, D.W, D.maxExt, D.maxRemote, D.ring,
                              D.slotRow.get(), D.padRow.get(), (const int4*)(back ? D.recUpCol.get() : D.recLoCol.get()),
                              KIND == kPartFactor ? D.prod.get() : back ? D.coefUp.get() : D.coefLo.get(),
                              back ? D.upRemote.get() : D.loRemote.get(), back ? D.upBox.get() : D.loBox.get(),
-                             D.coefLo.get(), D.coefUp.get(), D.ws.get(), src, w, D.psync.get(), D.nSteps, polls,
-                             D.err.get(), st,
+                             D.coefLo.get(), D.coefUp.get(), D.ws.get(), src, w, D.psync.get(), limit, D.err.get(), st,
                              int(kFlagDone)};
         VLM_LAUNCH_SMEM(k_dilu_pipe<KIND>, D.nParts, kPartThreads, D.partSmem, stream_, A);
         return;
@@ -1670,7 +1670,7 @@ void DeviceBatch::launchDiluPart(const double* src, double* w, const SysState* s
                          back ? D.upMail.get() : D.loMail.get(),
                          KIND == kPartFactor ? D.prod.get() : back ? D.coefUp.get() : D.coefLo.get(),
                          back ? D.upBox.get() : D.loBox.get(), D.rDs.get(), D.ws.get(), src, w, D.psync.get(),
-                         D.nSteps, polls, D.err.get(), st, int(kFlagDone)};
+                         limit, D.err.get(), st, int(kFlagDone)};
     if (D.local)
         VLM_LAUNCH_SMEM((k_dilu_part<KIND, true>), D.nParts, kPartThreads, D.partSmem, stream_, A);
     else
