@@ -294,3 +294,22 @@ def test_mailbox_wait_grows_with_the_steps_before_it(monkeypatch):
     monkeypatch.setenv("VLM_MAIL_POLLS", "1000")
     w = vb.precond_apply(vb.Mesh.from_arrays(msh), diag, upper, None, r, "DILU")
     assert np.array_equal(w, ro.precond_apply(msh, diag, upper, upper, r, "DILU"))
+
+
+@pytest.mark.parametrize("n", [(8, 7, 6), (44, 40, 36)])
+def test_gauss_seidel_before_dilu_on_one_mesh(n):
+    """Gauss-Seidel plans the levels alone; the sweeps' schedule follows with the first DILU call, and both
+    keep working on the mesh (one CTA, and parts)."""
+    from voluma_b200 import mesh as vm
+    msh = vm.box_mesh(n)
+    diag, upper = vm.poisson_matrix(msh)
+    r = np.random.default_rng(9).standard_normal(msh["n_cells"])
+    m = vb.Mesh.from_arrays(msh)
+    gs = vb.SolverControls("GaussSeidel", "none", 0.0, 1e-12, 4, nSweeps=2)
+    xo, _ = ro.solve(msh, diag, upper, None, r, np.zeros(msh["n_cells"]), "GaussSeidel", "none", 0.0, 1e-12, 4, n_sweeps=2)
+    for _ in range(2):
+        x = np.zeros(msh["n_cells"])
+        vb.solve_ldu(m, diag, upper, None, r, x, gs)
+        assert np.array_equal(x, xo)
+        w = vb.precond_apply(m, diag, upper, None, r, "DILU")
+        assert np.array_equal(w, ro.precond_apply(msh, diag, upper, upper, r, "DILU"))

@@ -21,8 +21,9 @@ namespace vlm {
 // the concatenated level table.
 struct DiluSys {
     int sys, levBegin, nLev, rowBegin, rowCount;  // rows [rowBegin, rowBegin + rowCount) of level 0
-    int slotBegin, slotEnd;                       // its slots: levRows[slotBegin .. slotEnd)
-    int loBegin, loEnd, upBegin, upEnd;           // its entries of the streamed schedule
+    // streamed schedule (addDiluStream): its slots levRows[slotBegin .. slotEnd), its entries
+    int slotBegin, slotEnd;
+    int loBegin, loEnd, upBegin, upEnd;
 };
 
 // One level of the streamed schedule: slots [s0, s0 + width) of levRows; entry j of slot s0 + q at
@@ -43,7 +44,7 @@ struct DiluPlan {
     // padding rows are on level 0 of their system
     std::vector<int32_t> levPtr, levRows;
     std::vector<DiluSys> sys;
-    // streamed schedule (per level of levPtr): slot -> row - rowBegin, entries (local column or -1,
+    // streamed schedule (addDiluStream; per level of levPtr): slot -> row - rowBegin, entries (local column or -1,
     // face as loFace)
     std::vector<DiluLevel> lev;
     std::vector<int32_t> slotRow;
@@ -59,6 +60,9 @@ int diluWidth(const DiluPlan& D, const DiluSys& ds, const BatchPlan& P);
 
 // systems: input order; P: the batch plan (solver order, perm0).
 DiluPlan buildDiluPlan(const std::vector<SysTopo>& systems, const BatchPlan& P);
+
+// Fills in the streamed schedule (systems whose sweeps run on one CTA each).
+void addDiluStream(DiluPlan& D);
 
 // Pipelined schedule of systems too wide for one CTA: the rows of a system are cut into parts of
 // consecutive natural rows, one CTA each.  A lower neighbour precedes its row in natural order, so a

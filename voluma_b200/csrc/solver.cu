@@ -32,12 +32,13 @@ struct DiluDev {
     DBuf<int> err;
     int G = 1, groups = 0;  // Gauss-Seidel sweeps: CTAs per system
     bool groupSweeps = false;  // a cooperative (G > 1) sweep has been recorded
+    bool sweeps = false;       // what follows is there: the DIC/DILU sweeps' schedule
     // streamed shared-memory sweeps (dilu.h DiluLevel): used when smem > 0
     DBuf<DiluLevel> lev;
     DBuf<int32_t> slotRow, sLoCol, sLoFace, sUpCol, sUpFace;
     DBuf<double> prod, coefLo, coefUp, rDs;
     int W = 0, M = 0, nLoS = 0, nUpS = 0;
-    size_t smem = 0;   // > 0: shared-memory sweeps with this many bytes per CTA
+    size_t smem = 0;   // > 0: shared-memory sweeps with this many bytes per CTA (known with the levels)
     int threads = 0;   // their CTA size: the widest level rounded up to whole warps (cheap barriers)
     // pipelined parts (dilupart.cuh): used otherwise; their entries are sLo* / sUp* above
     DBuf<DiluPart> parts;
@@ -439,7 +440,7 @@ bool DeviceBatch::levelScheduleInSharedMemory(const vlm_solver_ctrl& ctrl) {
     const bool levels = pk == PrecondKind::DIC || pk == PrecondKind::DILU || sk == SolverKind::GaussSeidel ||
                         sk == SolverKind::SymGaussSeidel;
     if (!levels) return true;
-    ensureDilu();
+    ensureDilu(false);
     return dilu_->smem > 0;
 }
 
@@ -1540,33 +1541,49 @@ void DeviceBatch::planDiluParts(DiluDev& D, const DiluPlan& P, int sms) {
     VLM_CUDA(cudaStreamSynchronize(s));  // R and C are locals
 }
 
-void DeviceBatch::ensureDilu() {
-    if (dilu_) return;
-    const DiluPlan P = buildDiluPlan(topo_, plan_);
-    auto D = std::make_unique<DiluDev>();
+// Opt-in shared memory of the one-CTA sweeps.
+constexpr size_t kDiluSmemMax = 200 * 1024;
+
+// The level schedule, and with `sweeps` what the DIC/DILU sweeps need besides (Gauss-Seidel has no use
+// for it: the parts take about 160 bytes a row).
+void DeviceBatch::ensureDilu(bool sweeps) {
+    if (dilu_ && (dilu_->sweeps || !sweeps)) return;
+    DiluPlan P = buildDiluPlan(topo_, plan_);
     cudaStream_t s = stream_;
-    D->levPtr.upload(P.levPtr, s);
-    D->levRows.upload(P.levRows, s);
-    D->sys.upload(P.sys, s);
-    D->groups = int(P.sys.size());
     int dev = 0, sms = 0;
     VLM_CUDA(cudaGetDevice(&dev));
     VLM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    // Gauss-Seidel: one CTA per system; a single wide system gets a co-resident group of CTAs
-    D->G = 1;
-    if (D->groups == 1 && P.maxWidth > 2 * kDiluThreads) {
-        int per = 0;
-        VLM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_gs_sweep, kDiluThreads, 0));
-        D->G = std::max(1, std::min({(P.maxWidth + kDiluThreads - 1) / kDiluThreads, sms * std::max(1, per), sms}));
+    if (!dilu_) {
+        auto D = std::make_unique<DiluDev>();
+        D->levPtr.upload(P.levPtr, s);
+        D->levRows.upload(P.levRows, s);
+        D->sys.upload(P.sys, s);
+        D->groups = int(P.sys.size());
+        // Gauss-Seidel: one CTA per system; a single wide system gets a co-resident group of CTAs
+        D->G = 1;
+        if (D->groups == 1 && P.maxWidth > 2 * kDiluThreads) {
+            int per = 0;
+            VLM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_gs_sweep, kDiluThreads, 0));
+            D->G = std::max(1, std::min({(P.maxWidth + kDiluThreads - 1) / kDiluThreads, sms * std::max(1, per), sms}));
+        }
+        // shared-memory sweeps: one CTA per system, every level at most one row per thread, the vector
+        // of the largest system within the opt-in shared memory
+        D->W = std::max(1, P.maxWidth);
+        D->M = std::max(1, P.maxEnt);
+        const size_t streamSmem = dilu_stream_smem(P.maxRows, P.maxLevels, D->W, D->M);
+        if (D->G == 1 && P.maxWidth <= kDiluThreads && streamSmem <= kDiluSmemMax) D->smem = streamSmem;
+        D->bars.resize(size_t(D->groups));
+        D->bars.zero(s);
+        D->err.resize(1);
+        D->err.zero(s);
+        VLM_CUDA(cudaStreamSynchronize(s));
+        dilu_ = std::move(D);
     }
-    // shared-memory sweeps: one CTA per system, every level at most one row per thread, the vector
-    // of the largest system within the opt-in shared memory
-    // (the kernels' opt-in limit is a per-function setting shared by every mesh: it is raised once to
-    // the ceiling, never to one mesh's size)
-    constexpr size_t kDiluSmemMax = 200 * 1024;
-    const int W = std::max(1, P.maxWidth), M = std::max(1, P.maxEnt);
-    const size_t streamSmem = dilu_stream_smem(P.maxRows, P.maxLevels, W, M);
-    if (D->G == 1 && P.maxWidth <= kDiluThreads && streamSmem <= kDiluSmemMax) {
+    if (!sweeps) return;
+    DiluDev& D = *dilu_;
+    if (D.smem) {
+        // (the kernels' opt-in limit is a per-function setting shared by every mesh: it is raised once to
+        // the ceiling, never to one mesh's size)
         static const bool raised = [] {
             VLM_CUDA(cudaFuncSetAttribute(k_dilu_factor_stream, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           int(kDiluSmemMax)));
@@ -1575,33 +1592,28 @@ void DeviceBatch::ensureDilu() {
             return true;
         }();
         (void)raised;
-        D->smem = streamSmem;
-        D->threads = std::max(32, (P.maxWidth + 31) / 32 * 32);
-        D->W = W;
-        D->M = M;
-        D->lev.upload(P.lev, s);
-        D->slotRow.upload(P.slotRow, s);
-        D->sLoCol.upload(P.sLoCol, s);
-        D->sLoFace.upload(P.sLoFace, s);
-        D->sUpCol.upload(P.sUpCol, s);
-        D->sUpFace.upload(P.sUpFace, s);
-        D->nLoS = int(P.sLoCol.size());
-        D->nUpS = int(P.sUpCol.size());
-        D->rDs.resize(std::max<size_t>(P.slotRow.size(), 1));
+        addDiluStream(P);
+        D.sys.upload(P.sys, s);
+        D.threads = std::max(32, (P.maxWidth + 31) / 32 * 32);
+        D.lev.upload(P.lev, s);
+        D.slotRow.upload(P.slotRow, s);
+        D.sLoCol.upload(P.sLoCol, s);
+        D.sLoFace.upload(P.sLoFace, s);
+        D.sUpCol.upload(P.sUpCol, s);
+        D.sUpFace.upload(P.sUpFace, s);
+        D.nLoS = int(P.sLoCol.size());
+        D.nUpS = int(P.sUpCol.size());
+        D.rDs.resize(std::max<size_t>(P.slotRow.size(), 1));
     } else {
-        planDiluParts(*D, P, sms);
+        planDiluParts(D, P, sms);
     }
-    const size_t nLo = D->records ? 4 * size_t(D->nRecLo) : size_t(std::max(D->nLoS, 1));
-    const size_t nUp = D->records ? 4 * size_t(D->nRecUp) : size_t(std::max(D->nUpS, 1));
-    D->prod.resize(nLo);
-    D->coefLo.resize(nLo);
-    D->coefUp.resize(nUp);
-    D->bars.resize(size_t(D->groups));
-    D->bars.zero(s);
-    D->err.resize(1);
-    D->err.zero(s);
+    const size_t nLo = D.records ? 4 * size_t(D.nRecLo) : size_t(std::max(D.nLoS, 1));
+    const size_t nUp = D.records ? 4 * size_t(D.nRecUp) : size_t(std::max(D.nUpS, 1));
+    D.prod.resize(nLo);
+    D.coefLo.resize(nLo);
+    D.coefUp.resize(nUp);
     VLM_CUDA(cudaStreamSynchronize(s));
-    dilu_ = std::move(D);
+    D.sweeps = true;
 }
 
 namespace {
@@ -1925,7 +1937,7 @@ void DeviceBatch::solve(const double* diag, const double* upper, const double* l
     }
     const bool levelSchedule = pk == PrecondKind::DIC || pk == PrecondKind::DILU || sk == SolverKind::GaussSeidel ||
                                sk == SolverKind::SymGaussSeidel;
-    if (levelSchedule) ensureDilu();
+    if (levelSchedule) ensureDilu(pk == PrecondKind::DIC || pk == PrecondKind::DILU);
     const SmootherKind sm = parseSmoother(ctrl.smoother);
     Precision prec = Precision::FP64;
     if (eq(ctrl.precision, "mixed"))
@@ -2113,7 +2125,7 @@ void DeviceBatch::precondApply(const double* diag, const double* upper, const do
     }
     cudaStream_t s = stream_;
     const bool dilu = pk == PrecondKind::DIC || pk == PrecondKind::DILU;
-    if (dilu) ensureDilu();
+    if (dilu) ensureDilu(true);
     setupMatrix(diag, upper, lower, false, false);
     DevLevel& D0 = L_[0];
     const int n0 = D0.nrows;

@@ -222,7 +222,7 @@ private:
     template <class T> void buildTailTable(DBuf<TailLevel<T>>& out);
     void planTail();
     void buildChunkLists();
-    void ensureDilu();
+    void ensureDilu(bool sweeps);
     void planDiluParts(DiluDev& D, const DiluPlan& P, int sms);
     template <int KIND> void launchDiluPart(const double* src, double* w, const SysState* st);
     void recordDiluApply(const double* r, double* w);
