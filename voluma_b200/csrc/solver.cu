@@ -677,11 +677,11 @@ void DeviceBatch::setupMatrix(const double* diag, const double* upper, const dou
     }
     if (tailOn_ && tailSmem_) {
         // the shared-memory tail's value images of this solve's coarse levels
-        const int n64 = int(tailPart_[0].codes.size()), n32 = int(tailPart_[1].codes.size());
-        VLM_LAUNCH(k_tail_values<double>, nblk(n64), 256, s, n64, tailPart_[0].codes.get(), tail64_.get(),
+        const int n64 = int(tailImages_[0]->codes.size()), n32 = int(tailImages_[1]->codes.size());
+        VLM_LAUNCH(k_tail_values<double>, nblk(n64), 256, s, n64, tailImages_[0]->codes.get(), tail64_.get(),
                    tailVal64_.get());
         if (mixed && tail32_.size() != 0)
-            VLM_LAUNCH(k_tail_values<float>, nblk(n32), 256, s, n32, tailPart_[1].codes.get(), tail32_.get(),
+            VLM_LAUNCH(k_tail_values<float>, nblk(n32), 256, s, n32, tailImages_[1]->codes.get(), tail32_.get(),
                        tailVal32_.get());
     }
 }
@@ -977,17 +977,17 @@ void DeviceBatch::recordTail(const T* r0, T* x0, int flag, bool jacobi0) {
     if (tailSmem_) {
         // every operand in shared memory, one CTA or one cluster per system
         constexpr bool f32 = std::is_same<T, float>::value;
-        const TailSmem& Q = tailPart_[f32 ? 1 : 0];
+        const TailSmem& Q = *tailImages_[f32 ? 1 : 0];
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(unsigned(Q.systems) * unsigned(Q.cluster));
+        cfg.gridDim = dim3(unsigned(Q.parts.size()));
         cfg.blockDim = dim3(unsigned(kTailPartThreads));
-        cfg.dynamicSmemBytes = Q.bytes;
+        cfg.dynamicSmemBytes = tailBytes_[f32 ? 1 : 0];
         cfg.stream = stream_;
         cudaLaunchAttribute at[2];
         int na = 0;
-        if (Q.cluster > 1) {
+        if (tailCluster_ > 1) {
             at[na].id = cudaLaunchAttributeClusterDimension;
-            at[na].val.clusterDim.x = unsigned(Q.cluster);
+            at[na].val.clusterDim.x = unsigned(tailCluster_);
             at[na].val.clusterDim.y = 1;
             at[na].val.clusterDim.z = 1;
             ++na;
@@ -1005,7 +1005,7 @@ void DeviceBatch::recordTail(const T* r0, T* x0, int flag, bool jacobi0) {
                                         (const uint16_t*)Q.str.get(), tab, (const double*)inv_.get(), r0, x0,
                                         T(jacobiOmega_), (const SysState*)st_.get(), flag, jacobi0 ? 1 : 0));
         };
-        switch (Q.cluster) {
+        switch (tailCluster_) {
         case 8: launch(k_vcycle_tail_parts<T, 8>); break;
         case 4: launch(k_vcycle_tail_parts<T, 4>); break;
         case 2: launch(k_vcycle_tail_parts<T, 2>); break;
@@ -1048,6 +1048,45 @@ void DeviceBatch::recordTail(const T* r0, T* x0, int flag, bool jacobi0) {
     }
     ++tl_launches;
 }
+
+namespace {
+
+// Bytes of dynamic shared memory a CTA of k_vcycle_tail_parts may use (its static descriptor aside).
+int tailBudget() {
+    int dev = 0, optin = 0;
+    VLM_CUDA(cudaGetDevice(&dev));
+    VLM_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    return optin - int(sizeof(TailPart)) - 256;
+}
+
+// The opt-in limit is a per-function setting, raised once to what the kernels may use; returns how
+// many clusters of CL such CTAs the device holds at once.
+template <int CL>
+int tailClusters() {
+    static const int n = [] {
+        const int budget = tailBudget();
+        VLM_CUDA(cudaFuncSetAttribute(k_vcycle_tail_parts<double, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, budget));
+        VLM_CUDA(cudaFuncSetAttribute(k_vcycle_tail_parts<float, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, budget));
+        if (CL == 1) return 1 << 30;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(unsigned(CL));
+        cfg.blockDim = dim3(unsigned(kTailPartThreads));
+        cfg.dynamicSmemBytes = size_t(budget);
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = unsigned(CL);
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        int count = 0;
+        VLM_CUDA(cudaOccupancyMaxActiveClusters(&count, k_vcycle_tail_parts<double, CL>, &cfg));
+        return count;
+    }();
+    return n;
+}
+
+}  // namespace
 
 // Per system: the first level of the tail = the first level (below level 0) whose padded row count
 // is at most the row limit (VLM_TAIL_ROWS overrides; VLM_TAIL=0 disables), else the coarsest level
@@ -1120,9 +1159,11 @@ void DeviceBatch::planTail() {
         // at most one row per thread of one CTA on every level: its own barrier is shorter than the
         // cluster's (480 cells, 11 iterations: 0.65 -> 0.61 ms a solve).  Running only the levels below
         // 512 rows of a larger tail that way measured slower (96^3 FP64 11.26 -> 11.39 ms).
-        if (std::all_of(ts.begin(), ts.end(), [](const TailSys& t) { return t.rowCount[t.first] <= kTailPartThreads; }))
-            cluster = tailClusterFor(1 << 30);
-        tailSmem_ = planTailSmem<double>(ts, cluster) && planTailSmem<float>(ts, cluster);
+        if (std::all_of(ts.begin(), ts.end(), [](const TailSys& t) { return t.rowCount[t.first] <= kTailPartThreads; })) {
+            tailClusters<1>();
+            cluster = 1;
+        }
+        tailSmem_ = planTailSmem(ts, cluster);
     }
     if (!tailSmem_) {  // one CTA or a cluster of tailCl_ CTAs per system on global memory
         std::vector<TailSys> ts = starts(tailCl_);
@@ -1138,45 +1179,6 @@ void DeviceBatch::planTail() {
     tailOn_ = true;
 }
 
-namespace {
-
-// Bytes of dynamic shared memory a CTA of k_vcycle_tail_parts may use (its static descriptor aside).
-int tailBudget() {
-    int dev = 0, optin = 0;
-    VLM_CUDA(cudaGetDevice(&dev));
-    VLM_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    return optin - int(sizeof(TailPart)) - 256;
-}
-
-// The opt-in limit is a per-function setting, raised once to what the kernels may use; returns how
-// many clusters of CL such CTAs the device holds at once.
-template <int CL>
-int tailClusters() {
-    static const int n = [] {
-        const int budget = tailBudget();
-        VLM_CUDA(cudaFuncSetAttribute(k_vcycle_tail_parts<double, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, budget));
-        VLM_CUDA(cudaFuncSetAttribute(k_vcycle_tail_parts<float, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, budget));
-        if (CL == 1) return 1 << 30;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(unsigned(CL));
-        cfg.blockDim = dim3(unsigned(kTailPartThreads));
-        cfg.dynamicSmemBytes = size_t(budget);
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = unsigned(CL);
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        int count = 0;
-        VLM_CUDA(cudaOccupancyMaxActiveClusters(&count, k_vcycle_tail_parts<double, CL>, &cfg));
-        return count;
-    }();
-    return n;
-}
-
-}  // namespace
-
 int DeviceBatch::tailClusterFor(int systems) {
     if (systems <= tailClusters<8>()) return 8;
     if (systems <= tailClusters<4>()) return 4;
@@ -1185,26 +1187,31 @@ int DeviceBatch::tailClusterFor(int systems) {
     return 1;
 }
 
-// Images of the shared-memory tail in one precision (buildTailImages); false when a system's
-// coarsest level alone does not fit.
-template <class T>
-bool DeviceBatch::planTailSmem(std::vector<TailSys>& ts, int cluster) {
-    constexpr bool f32 = std::is_same<T, float>::value;
-    TailImages im;
-    if (!buildTailImages(plan_, ts, cluster, sizeof(T), size_t(tailBudget()), im)) return false;
-    TailSmem& Q = tailPart_[f32 ? 1 : 0];
-    Q.cluster = cluster;
-    Q.systems = int(ts.size());
-    Q.bytes = im.bytes;
-    Q.parts.upload(im.parts, stream_);
-    Q.codes.upload(im.codes, stream_);
-    Q.str.upload(im.str, stream_);
-    if (f32)
-        tailVal32_.resize(im.codes.size());
-    else
-        tailVal64_.resize(im.codes.size());
-    tailFirst_[f32 ? 1 : 0] = im.first;
-    VLM_CUDA(cudaStreamSynchronize(stream_));  // the host vectors are locals
+// Start levels and images of the shared-memory tail in both precisions; false when a system's coarsest
+// level alone does not fit.  The images hold structure and gather codes, so one copy serves both where
+// every tail starts at the same level (FP32 starts earlier only where FP64 does not fit).
+bool DeviceBatch::planTailSmem(const std::vector<TailSys>& ts, int cluster) {
+    for (int p = 0; p < 2; ++p)
+        if (!tailStarts(plan_, ts, cluster, p == 0 ? sizeof(double) : sizeof(float), size_t(tailBudget()), tailFirst_[p],
+                        tailBytes_[p]))
+            return false;
+    tailCluster_ = cluster;
+    for (int p = 0; p < 2; ++p) {
+        if (p == 1 && tailFirst_[1] == tailFirst_[0]) {
+            tailImages_[1] = tailImages_[0];
+            break;
+        }
+        TailImages im;
+        if (!buildTailImages(plan_, ts, tailFirst_[p], cluster, im)) return false;
+        auto Q = std::make_shared<TailSmem>();
+        Q->parts.upload(im.parts, stream_);
+        Q->codes.upload(im.codes, stream_);
+        Q->str.upload(im.str, stream_);
+        VLM_CUDA(cudaStreamSynchronize(stream_));  // the host vectors are locals
+        tailImages_[p] = std::move(Q);
+    }
+    tailVal64_.resize(tailImages_[0]->codes.size());
+    tailVal32_.resize(tailImages_[1]->codes.size());
     return true;
 }
 

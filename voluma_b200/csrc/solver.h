@@ -278,15 +278,16 @@ private:
     // shared-memory tail (k_vcycle_tail_parts): used when every system's coarsest levels fit
     bool tailSmem_ = false, tailSmemAllowed_ = true;
     struct TailSmem {
-        int cluster = 1, systems = 0;
-        size_t bytes = 0;                // dynamic shared memory per CTA
         DBuf<TailPart> parts;
         DBuf<int32_t> codes;             // value-image gather codes (k_tail_values)
         DBuf<uint16_t> str;              // structure images
-    } tailPart_[2];
+    };
+    std::shared_ptr<TailSmem> tailImages_[2];  // per precision; one and the same where the tails start alike
+    size_t tailBytes_[2] = {0, 0};       // dynamic shared memory per CTA
+    int tailCluster_ = 1;                // CTAs of a system's cluster
     DBuf<double> tailVal64_;
     DBuf<float> tailVal32_;
-    template <class T> bool planTailSmem(std::vector<TailSys>& ts, int cluster);
+    bool planTailSmem(const std::vector<TailSys>& ts, int cluster);
     int tailClusterFor(int systems);
     int tailCl_ = 1;                     // > 1: CTAs of the global-memory tail's cluster (asked for by setTail)
     int64_t tailMaxRows_ = 0;            // levels of at most this many rows go to the tail (0: scaled default)

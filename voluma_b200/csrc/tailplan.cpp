@@ -10,39 +10,83 @@ namespace vlm {
 
 namespace {
 
-// One system's parts from level f on, appended to `out`; false (and nothing appended) when they do not fit.
-bool appendSystem(const BatchPlan& plan, const TailSys& s, int f, int CL, size_t tsize, size_t budget, TailImages& out) {
-    const int c = s.coarsest;
-    if (c >= kTailMaxLevels || c > 31) return false;
-    int vec = 0;
-    int n[kTailMaxLevels], tX[kTailMaxLevels], tX2[kTailMaxLevels], tR[kTailMaxLevels] = {};
-    for (int k = f; k <= c; ++k) {
-        n[k] = s.rowCount[k];
-        if (n[k] >= 0xffff || n[k] % kSlice != 0 || s.rowStart[k] % kSlice != 0) return false;
-        tX[k] = vec;
-        tX2[k] = vec + n[k];
-        vec += 2 * n[k];
-        if (k < c) {
-            tR[k] = vec;
-            vec += (n[k] / kSlice + CL - 1) / CL * kSlice;
+// Where one system's vectors lie in every part's shared memory, levels f on.
+struct Vectors {
+    int count = 0;
+    int n[kTailMaxLevels] = {}, tX[kTailMaxLevels] = {}, tX2[kTailMaxLevels] = {}, tR[kTailMaxLevels] = {};
+
+    Vectors(const TailSys& s, int f, int CL) {
+        for (int k = f; k <= s.coarsest; ++k) {
+            n[k] = s.rowCount[k];
+            tX[k] = count;
+            tX2[k] = count + n[k];
+            count += 2 * n[k];
+            if (k < s.coarsest) {
+                tR[k] = count;
+                count += (n[k] / kSlice + CL - 1) / CL * kSlice;
+            }
         }
+        count = (count + 3) & ~3;  // whole 16-byte words in both precisions
     }
-    vec = (vec + 3) & ~3;  // whole 16-byte words in both precisions
-    if (s.coarseN > n[c]) return false;
-    if (size_t(vec) * tsize > budget) return false;
+    // rows of level k that part `rank` holds
+    int rows(int k, int rank, int CL) const {
+        const int ns = n[k] / kSlice;
+        return ns > rank ? (ns - rank + CL - 1) / CL * kSlice : 0;
+    }
+};
+
+// Largest part of system s from level f on, in bytes of shared memory; 0 when the parts do not fit `budget`
+// or their indices 16 bits.  Nothing is built for a level that does not fit.
+size_t partBytes(const BatchPlan& plan, const TailSys& s, int f, int CL, size_t tsize, size_t budget) {
+    const int c = s.coarsest;
+    if (c >= kTailMaxLevels || c > 31) return 0;
+    for (int k = f; k <= c; ++k)
+        if (s.rowCount[k] >= 0xffff || s.rowCount[k] % kSlice != 0 || s.rowStart[k] % kSlice != 0) return 0;
+    if (s.coarseN > s.rowCount[c]) return 0;
+    const Vectors v(s, f, CL);
+    if (size_t(v.count) * tsize > budget) return 0;
     for (int k = f; k < c; ++k) {
         const LevelPlan& P = plan.levels[k];
-        if (P.col.empty() || P.rlen.size() < size_t(s.rowStart[k] + n[k])) return false;  // host structure released
+        if (P.col.empty() || P.rlen.size() < size_t(s.rowStart[k] + v.n[k])) return 0;  // host structure released
+        if (s.rowStart[k] + v.n[k] > (1 << 25) || P.slPtr[size_t((s.rowStart[k] + v.n[k]) / kSlice)] >= (1 << 25)) return 0;
     }
-    const size_t nParts = out.parts.size(), nCodes = out.codes.size(), nStr = out.str.size();
-    auto fail = [&] {
-        out.parts.resize(nParts);
-        out.codes.resize(nCodes);
-        out.str.resize(nStr);
-        return false;
-    };
-    const int invRows = (s.coarseN + CL - 1) / CL;
-    size_t largest = out.bytes;
+    if (f == 0 && c > 0)
+        for (int q = 0; q < s.nColours; ++q)
+            if ((s.grpStart[q] - s.rowStart[0]) % kSlice != 0 || s.grpCount[q] % kSlice != 0) return 0;
+    size_t largest = 0;
+    for (int rank = 0; rank < CL; ++rank) {
+        size_t val = 0, str = 0;
+        for (int k = f; k < c; ++k) {
+            const LevelPlan& P = plan.levels[k];
+            const int nl = v.rows(k, rank, CL), nl1 = v.rows(k + 1, rank, CL);
+            size_t ent = 0, kids = 0;
+            for (int l = 0; l < nl; l += kSlice) {
+                const size_t sl = size_t(s.rowStart[k] / kSlice + l / kSlice * CL + rank);
+                ent += size_t(P.slPtr[sl + 1] - P.slPtr[sl]);
+            }
+            for (int l = 0; l < nl1; l += kSlice) {
+                const size_t R = size_t(s.rowStart[k + 1] + (l / kSlice * CL + rank) * kSlice);
+                kids += size_t(P.childPtr[R + kSlice] - P.childPtr[R]);
+            }
+            if (ent / kSlice > 0xffff || kids > 0xffff) return 0;
+            val += size_t(nl) + ent;
+            str += 2 * size_t(nl) + size_t(nl / kSlice) + ent + size_t(nl1) + 1 + kids;
+        }
+        val = (val + 3) & ~size_t(3);
+        str = (str + 7) & ~size_t(7);
+        const size_t inv = size_t(s.coarseN) * size_t((s.coarseN + CL - 1) / CL);
+        if ((size_t(v.count) + val) * tsize > budget || str * sizeof(uint16_t) > budget) return 0;
+        const size_t bytes = tail_smem_bytes(tsize, int(size_t(v.count) + val), int(inv), int(str));
+        if (bytes > budget) return 0;
+        largest = std::max(largest, bytes);
+    }
+    return largest;
+}
+
+// One system's parts from level f on, appended to `out`; false when the plan's indices are inconsistent.
+bool appendSystem(const BatchPlan& plan, const TailSys& s, int f, int CL, TailImages& out) {
+    const int c = s.coarsest;
+    const Vectors v(s, f, CL);
     for (int rank = 0; rank < CL; ++rank) {
         TailPart I;
         std::memset(&I, 0, sizeof I);
@@ -51,23 +95,21 @@ bool appendSystem(const BatchPlan& plan, const TailSys& s, int f, int CL, size_t
         I.coarsest = c;
         I.nc = s.coarseN;
         I.invOffset = s.invOffset;
-        I.vecCount = vec;
+        I.vecCount = v.count;
         I.two = s.two;
         I.nColours = s.nColours;
         if (f == 0 && c > 0)
             for (int q = 0; q < s.nColours; ++q) {
                 I.grpStart[q] = s.grpStart[q] - s.rowStart[0];
                 I.grpCount[q] = s.grpCount[q];
-                if (I.grpStart[q] % kSlice != 0 || I.grpCount[q] % kSlice != 0) return fail();
             }
         for (int k = f; k <= c; ++k) {
-            I.n[k] = n[k];
+            I.n[k] = v.n[k];
             I.rowStart[k] = s.rowStart[k];
-            const int ns = n[k] / kSlice;
-            I.nl[k] = ns > rank ? (ns - rank + CL - 1) / CL * kSlice : 0;
-            I.tX[k] = tX[k];
-            I.tX2[k] = tX2[k];
-            I.tR[k] = tR[k];
+            I.nl[k] = v.rows(k, rank, CL);
+            I.tX[k] = v.tX[k];
+            I.tX2[k] = v.tX2[k];
+            I.tR[k] = v.tR[k];
         }
         // value image: per level the diagonal of this CTA's rows, then its slices' entries
         I.valOff = int(out.codes.size());
@@ -75,27 +117,23 @@ bool appendSystem(const BatchPlan& plan, const TailSys& s, int f, int CL, size_t
         for (int k = f; k < c; ++k) {
             const LevelPlan& P = plan.levels[k];
             const int slice0 = s.rowStart[k] / kSlice;
-            I.tDiag[k] = vec + tc;
-            for (int l = 0; l < I.nl[k]; l += kSlice)
-                for (int i = 0; i < kSlice; ++i) {
-                    const int row = s.rowStart[k] + (l / kSlice * CL + rank) * kSlice + i;
-                    if (row >= (1 << 25)) return fail();
-                    out.codes.push_back((k << 26) | (1 << 25) | row);
-                }
+            I.tDiag[k] = v.count + tc;
+            for (int l = 0; l < I.nl[k]; l += kSlice) {
+                const int row = s.rowStart[k] + (l / kSlice * CL + rank) * kSlice;
+                for (int i = 0; i < kSlice; ++i) out.codes.push_back((k << 26) | (1 << 25) | (row + i));
+            }
             tc += I.nl[k];
-            I.tVal[k] = vec + tc;
+            I.tVal[k] = v.count + tc;
             for (int l = 0; l < I.nl[k]; l += kSlice) {
                 const int sl = slice0 + l / kSlice * CL + rank;
                 const int e0 = P.slPtr[size_t(sl)], e1 = P.slPtr[size_t(sl) + 1];
-                if (e1 >= (1 << 25)) return fail();
-                for (int e = e0; e < e1; ++e) {
-                    const int q = (e - e0) / kSlice;
-                    const bool real = q < P.rlen[size_t(sl * kSlice + (e - e0) % kSlice)];
-                    out.codes.push_back(real ? (k << 26) | e : -1);
-                }
+                const int32_t* rlen = P.rlen.data() + size_t(sl) * kSlice;
+                out.codes.resize(out.codes.size() + size_t(e1 - e0));
+                int32_t* w = out.codes.data() + out.codes.size() - size_t(e1 - e0);
+                for (int e = e0, q = 0; e < e1; e += kSlice, ++q, w += kSlice)
+                    for (int i = 0; i < kSlice; ++i) w[i] = q < rlen[i] ? (k << 26) | (e + i) : -1;
                 tc += e1 - e0;
             }
-            if (size_t(vec + tc) * tsize > budget) return fail();
         }
         while (tc % 4) {
             out.codes.push_back(-1);
@@ -104,85 +142,92 @@ bool appendSystem(const BatchPlan& plan, const TailSys& s, int f, int CL, size_t
         I.valCount = tc;
         // structure image: row lengths, slice offsets, level-local columns, aggregates, children
         I.strOff = int(out.str.size());
-        int su = 0;
-        bool fits = true;
-        auto push = [&](int v) {
-            if (v < 0 || v > 0xffff) fits = false;
-            out.str.push_back(uint16_t(v));
-            ++su;
-        };
+        const size_t str0 = out.str.size();
+        auto at = [&] { return int(out.str.size() - str0); };
+        auto push = [&](int w) { out.str.push_back(uint16_t(w)); };
         for (int k = f; k < c; ++k) {
             const LevelPlan& P = plan.levels[k];
             const int rs = s.rowStart[k], slice0 = rs / kSlice, rs1 = s.rowStart[k + 1];
             auto row = [&](int l) { return rs + (l / kSlice * CL + rank) * kSlice + l % kSlice; };
-            I.uRlen[k] = su;
+            I.uRlen[k] = at();
             for (int l = 0; l < I.nl[k]; ++l) push(P.rlen[size_t(row(l))]);
-            I.uSlice[k] = su;
+            I.uSlice[k] = at();
             int off = 0;
             for (int l = 0; l < I.nl[k]; l += kSlice) {
                 push(off);
                 const int sl = slice0 + l / kSlice * CL + rank;
                 off += (P.slPtr[size_t(sl) + 1] - P.slPtr[size_t(sl)]) / kSlice;
             }
-            I.uCol[k] = su;
+            I.uCol[k] = at();
             for (int l = 0; l < I.nl[k]; l += kSlice) {
                 const int sl = slice0 + l / kSlice * CL + rank;
                 const int e0 = P.slPtr[size_t(sl)], e1 = P.slPtr[size_t(sl) + 1];
-                for (int e = e0; e < e1; ++e) {
-                    int cl = 0;
-                    if ((e - e0) / kSlice < P.rlen[size_t(sl * kSlice + (e - e0) % kSlice)]) {
-                        cl = P.col[size_t(e)] - rs;
-                        if (cl < 0 || cl >= n[k]) return fail();
+                const int32_t* rlen = P.rlen.data() + size_t(sl) * kSlice;
+                out.str.resize(out.str.size() + size_t(e1 - e0));
+                uint16_t* w = out.str.data() + out.str.size() - size_t(e1 - e0);
+                const int32_t* col = P.col.data() + e0;
+                bool ok = true;
+                for (int e = e0, q = 0; e < e1; e += kSlice, ++q, w += kSlice, col += kSlice)
+                    for (int i = 0; i < kSlice; ++i) {
+                        const int cl = q < rlen[i] ? col[i] - rs : 0;
+                        ok = ok && cl >= 0 && cl < v.n[k];
+                        w[i] = uint16_t(cl);
                     }
-                    push(cl);
-                }
+                if (!ok) return false;
             }
-            I.uAgg[k] = su;
+            I.uAgg[k] = at();
             for (int l = 0; l < I.nl[k]; ++l) {
                 const int a = P.agg[size_t(row(l))];
-                if (a >= 0 && (a - rs1 < 0 || a - rs1 >= n[k + 1])) return fail();
+                if (a >= 0 && (a - rs1 < 0 || a - rs1 >= v.n[k + 1])) return false;
                 push(a < 0 ? 0xffff : a - rs1);
             }
             // children of this CTA's rows of the next level
             auto crow = [&](int l) { return rs1 + (l / kSlice * CL + rank) * kSlice + l % kSlice; };
-            I.uCptr[k] = su;
+            I.uCptr[k] = at();
             int cnt = 0;
             push(0);
             for (int l = 0; l < I.nl[k + 1]; ++l) {
                 cnt += P.childPtr[size_t(crow(l)) + 1] - P.childPtr[size_t(crow(l))];
                 push(cnt);
             }
-            I.uChild[k] = su;
+            I.uChild[k] = at();
             for (int l = 0; l < I.nl[k + 1]; ++l)
                 for (int q = P.childPtr[size_t(crow(l))]; q < P.childPtr[size_t(crow(l)) + 1]; ++q) {
-                    const int v = P.child[size_t(q)] - rs;
-                    if (v < 0 || v >= n[k]) return fail();
-                    push(v);
+                    const int w = P.child[size_t(q)] - rs;
+                    if (w < 0 || w >= v.n[k]) return false;
+                    push(w);
                 }
         }
-        while (su % 8) push(0);
-        I.strCount = su;
-        const size_t bytes = tail_smem_bytes(tsize, vec + tc, s.coarseN * invRows, su);
-        if (!fits || bytes > budget) return fail();
-        largest = std::max(largest, bytes);
+        while (at() % 8) push(0);
+        I.strCount = at();
         out.parts.push_back(I);
     }
-    out.bytes = largest;
     return true;
 }
 
 }  // namespace
 
-bool buildTailImages(const BatchPlan& plan, const std::vector<TailSys>& ts, int cluster, size_t tsize, size_t budget,
-                     TailImages& out) {
-    out = TailImages();
+bool tailStarts(const BatchPlan& plan, const std::vector<TailSys>& ts, int cluster, size_t tsize, size_t budget,
+                std::vector<int>& first, size_t& bytes) {
+    first.clear();
+    bytes = 0;
     for (const TailSys& s : ts) {
         int f = s.first;
-        while (f <= s.coarsest && !appendSystem(plan, s, f, cluster, tsize, budget, out)) ++f;
+        size_t b = 0;
+        while (f <= s.coarsest && (b = partBytes(plan, s, f, cluster, tsize, budget)) == 0) ++f;
         if (f > s.coarsest) return false;
-        out.first.push_back(f);
+        first.push_back(f);
+        bytes = std::max(bytes, b);
     }
     return !ts.empty();
+}
+
+bool buildTailImages(const BatchPlan& plan, const std::vector<TailSys>& ts, const std::vector<int>& first, int cluster,
+                     TailImages& out) {
+    out = TailImages();
+    for (size_t b = 0; b < ts.size(); ++b)
+        if (!appendSystem(plan, ts[b], first[b], cluster, out)) return false;
+    return true;
 }
 
 }  // namespace vlm
