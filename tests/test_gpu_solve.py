@@ -362,6 +362,34 @@ def test_tail_launch_configurations_give_identical_results(name, precision):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("shape,auto", [((20, 20, 20), 8), ((9, 7, 5), 1)])
+def test_tail_width_can_be_asked_for(shape, auto, monkeypatch):
+    """The planner's width is reported, every width can be asked for, in shared and in global memory, and
+    none changes the solution; 0 keeps the width that was asked for."""
+    M = vm.box_mesh(shape)
+    d, up = vm.poisson_matrix(M)
+    b = np.random.default_rng(4).standard_normal(M["n_cells"])
+    c = ctrl(preconditioner="GAMG")
+    monkeypatch.setenv("VLM_TUNE", "0")
+    ref = None
+    for smem in ("1", "0"):
+        monkeypatch.setenv("VLM_TAIL_SMEM", smem)
+        m = vb.Mesh.from_arrays(M)
+        assert m.tail_config() == ((auto if smem == "1" else 1), 0, 0)
+        for cluster in (0, 1, 2, 4, 8, 0):
+            m.set_tail(cluster)
+            if cluster:
+                assert m.tail_config() == (cluster, 0, 0)
+            x = np.zeros(M["n_cells"])
+            p = vb.solve_ldu(m, d, up, None, b, x, c)
+            if ref is None:
+                ref = (x, p.iterations)
+            assert p.iterations == ref[1] and np.array_equal(x, ref[0]), (smem, cluster)
+        assert m.tail_config() == (8, 0, 0)
+        m.close()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("name", ["periodic24", "stretched6x9x5"])
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 def test_fused_coarse_launches_give_identical_results(name, precision):

@@ -287,11 +287,12 @@ class Mesh:
 
     def set_tail(self, cluster: int = 0, max_rows: int = 0, full_rows: int = 0):
         """Coarse V-cycle tail launch configuration (vlm_mesh_set_tail): cluster size 1/2/4/8, level
-        row limit, whole-V-cycle row limit; 0 keeps a value.  Results are unchanged bit for bit."""
+        row limit, whole-V-cycle row limit; 0 keeps a value (the planner picks a cluster that was never
+        set).  Results are unchanged bit for bit."""
         check(load().vlm_mesh_set_tail(self._h, int(cluster), int(max_rows), int(full_rows)), self.ctx.handle)
 
     def tail_config(self):
-        """(cluster, max_rows, full_rows) of the coarse tail; row limits 0 = scaled defaults."""
+        """(cluster, max_rows, full_rows) of the coarse tail: the cluster in use; row limits 0 = scaled defaults."""
         c, a, b = C.c_int32(), C.c_int64(), C.c_int64()
         check(load().vlm_mesh_get_tail(self._h, C.byref(c), C.byref(a), C.byref(b)))
         return c.value, a.value, b.value

@@ -376,8 +376,6 @@ void DeviceBatch::buildChunkLists() {
     }
 }
 
-// Re-plans the coarse tail (cluster size, level row limit, whole-V-cycle row limit; 0 keeps the
-// current value) on a registered batch: chunk lists, tail tables, and the recorded graphs.
 // Row limits of the fused coarse-level launches (negative keeps a value); the recorded graphs go.
 void DeviceBatch::setFusion(int64_t pre, int64_t restrict, int64_t post) {
     VLM_CUDA(cudaStreamSynchronize(stream_));
@@ -387,6 +385,8 @@ void DeviceBatch::setFusion(int64_t pre, int64_t restrict, int64_t post) {
     graphs_.clear();
 }
 
+// Re-plans the coarse tail (cluster size, level row limit, whole-V-cycle row limit; 0 keeps the
+// current value) on a registered batch: chunk lists, tail tables, and the recorded graphs.
 void DeviceBatch::setTail(int cluster, int64_t maxRows, int64_t fullRows) {
     if (cluster != 0) tailCl_ = cluster;
     if (maxRows != 0) tailMaxRows_ = maxRows;
@@ -1014,16 +1014,16 @@ void DeviceBatch::recordTail(const T* r0, T* x0, int flag, bool jacobi0) {
         ++tl_launches;
         return;
     }
-    // one CTA, or one thread-block cluster of tailCl_ CTAs, per system
+    // one CTA, or one thread-block cluster, per system
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(unsigned(tailSys_.size()) * unsigned(tailCl_));
+    cfg.gridDim = dim3(unsigned(tailSys_.size()) * unsigned(tailCluster_));
     cfg.blockDim = dim3(unsigned(kTailThreads));
     cfg.stream = stream_;
     cudaLaunchAttribute at[2];
     int na = 0;
-    if (tailCl_ > 1) {
+    if (tailCluster_ > 1) {
         at[na].id = cudaLaunchAttributeClusterDimension;
-        at[na].val.clusterDim.x = unsigned(tailCl_);
+        at[na].val.clusterDim.x = unsigned(tailCluster_);
         at[na].val.clusterDim.y = 1;
         at[na].val.clusterDim.z = 1;
         ++na;
@@ -1039,7 +1039,7 @@ void DeviceBatch::recordTail(const T* r0, T* x0, int flag, bool jacobi0) {
         VLM_CUDA(cudaLaunchKernelEx(&cfg, kernel, (const TailSys*)tailSys_.get(), tab, (const double*)inv_.get(), r0, x0,
                                     T(jacobiOmega_), (const SysState*)st_.get(), flag, jacobi0 ? 1 : 0));
     };
-    switch (tailCl_) {
+    switch (tailCluster_) {
     case 1: launch(k_vcycle_tail<T, 1>); break;
     case 2: launch(k_vcycle_tail<T, 2>); break;
     case 4: launch(k_vcycle_tail<T, 4>); break;
@@ -1090,16 +1090,16 @@ int tailClusters() {
 
 // Per system: the first level of the tail = the first level (below level 0) whose padded row count
 // is at most the row limit (VLM_TAIL_ROWS overrides; VLM_TAIL=0 disables), else the coarsest level
-// alone; the whole V-cycle for systems of at most the full-row limit.  Without a wider global-memory
-// cluster asked for, the tail runs in shared memory on one cluster per system, as wide as lets
-// every system's cluster be resident at once (tailClusterFor), and the limits scale with that width:
-// a level has at most one row per thread of the cluster.
+// alone; the whole V-cycle for systems of at most the full-row limit.  The tail runs in shared memory on
+// one cluster per system: of the width asked for, else as wide as lets every system's cluster be
+// resident at once (tailClusterFor); in global memory where the coarsest levels do not fit.  Limits that
+// are not set scale with the width.
 void DeviceBatch::planTail() {
     const char* tv = std::getenv("VLM_TAIL");
     if (tv && tv[0] == '0') return;
     const int ns = plan_.nsys;
     if (ns == 0) return;
-    if (tailCl_ != 1 && tailCl_ != 2 && tailCl_ != 4 && tailCl_ != 8)
+    if (tailCl_ != 0 && tailCl_ != 1 && tailCl_ != 2 && tailCl_ != 4 && tailCl_ != 8)
         throw Error(VLM_ERR_BAD_ARG, "the coarse-tail cluster size must be 1, 2, 4 or 8");
     const LevelPlan& L0 = plan_.levels[0];
     auto starts = [&](int cluster) {
@@ -1153,7 +1153,11 @@ void DeviceBatch::planTail() {
         return ts;
     };
     tailSmem_ = false;
-    if (tailSmemAllowed_ && tailCl_ == 1) {
+    if (tailSmemAllowed_ && tailCl_ != 0) {
+        const int resident = tailCl_ == 8 ? tailClusters<8>() : tailCl_ == 4 ? tailClusters<4>()
+                             : tailCl_ == 2 ? tailClusters<2>() : tailClusters<1>();
+        tailSmem_ = resident > 0 && planTailSmem(starts(tailCl_), tailCl_);
+    } else if (tailSmemAllowed_) {
         int cluster = tailClusterFor(ns);
         std::vector<TailSys> ts = starts(cluster);
         // at most one row per thread of one CTA on every level: its own barrier is shorter than the
@@ -1165,8 +1169,9 @@ void DeviceBatch::planTail() {
         }
         tailSmem_ = planTailSmem(ts, cluster);
     }
-    if (!tailSmem_) {  // one CTA or a cluster of tailCl_ CTAs per system on global memory
-        std::vector<TailSys> ts = starts(tailCl_);
+    if (!tailSmem_) {  // one CTA, or the cluster asked for, per system on global memory
+        tailCluster_ = std::max(tailCl_, 1);
+        std::vector<TailSys> ts = starts(tailCluster_);
         for (int p = 0; p < 2; ++p) {
             tailFirst_[p].clear();
             for (const TailSys& t : ts) tailFirst_[p].push_back(t.first);

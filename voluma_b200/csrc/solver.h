@@ -163,7 +163,7 @@ public:
         *post = fusePost_;
     }
     void tailConfig(int* cluster, int64_t* maxRows, int64_t* fullRows) const {
-        *cluster = tailCl_;
+        *cluster = tailCl_ != 0 ? tailCl_ : tailCluster_;
         *maxRows = tailMaxRows_;
         *fullRows = tailFullRows_;
     }
@@ -289,7 +289,7 @@ private:
     DBuf<float> tailVal32_;
     bool planTailSmem(const std::vector<TailSys>& ts, int cluster);
     int tailClusterFor(int systems);
-    int tailCl_ = 1;                     // > 1: CTAs of the global-memory tail's cluster (asked for by setTail)
+    int tailCl_ = 0;                     // CTAs of the tail's cluster asked for (setTail); 0: planTail picks
     int64_t tailMaxRows_ = 0;            // levels of at most this many rows go to the tail (0: scaled default)
     int64_t tailFullRows_ = 0;           // systems of at most this many level-0 rows: whole V-cycle there
     // fused coarse-level launches on levels of at most this many rows (all systems): both Jacobi

@@ -2,18 +2,20 @@
 
 The knob it tunes is where the V-cycle switches from per-level launches (a few kernels per level,
 each spread over the whole GPU) to the coarse tail (all remaining levels of a system in one launch
-on a thread-block cluster, steps separated by the cluster barrier), and how wide that cluster is:
+on a thread-block cluster, in its shared memory, steps separated by the cluster barrier), and how wide
+that cluster is:
 
-* cluster   - CTAs per system in the tail launch: 1, 2, 4 or 8 (1024 threads each);
+* cluster   - CTAs per system in the tail launch: 1, 2, 4 or 8 (512 threads each);
 * max_rows  - levels of at most this many rows go to the tail;
 * full_rows - systems of at most this many level-0 rows run their whole V-cycle in the tail.
 
 None of them changes a result: the tail performs the same row operations in the same order.  For a
 mesh, every configuration that splits its levels differently is timed with CUDA events on full
-GAMG-PCG solves (the production path: one graph launch per solve), and the fastest is kept.  The
-results go to a per-device table (voluma_b200/tuning/<device>.json, one entry per mesh-size class:
-level-0 rows and number of systems), which Mesh registration applies to every new mesh of the same
-device (Mesh._apply_tuning: nearest size class, same single/batched kind).
+GAMG-PCG solves (the production path: one graph launch per solve); the fastest is kept where it beats the
+built-in choice by more than MARGIN, the spread of such medians.  The results go to a per-device table (voluma_b200/tuning/<device>.json, one entry per mesh-size class:
+level-0 rows and number of systems; "default" where the built-in choice stays), which Mesh registration
+applies to every new mesh of the same device (Mesh._apply_tuning: nearest size class, same single/batched
+kind).
 
     python -m voluma_b200.tune [--out voluma_b200/tuning] [--cases tgv128,tgv64,...]
 """
@@ -30,6 +32,7 @@ import numpy as np
 HERE = os.path.dirname(os.path.abspath(__file__))
 TABLE_DIR = os.path.join(HERE, "tuning")
 _tables: dict = {}
+MARGIN = 0.02
 
 
 def _slug(name: str) -> str:
@@ -63,12 +66,13 @@ def lookup(entries: list, rows0: int, nsys: int):
 
 
 def apply(mesh) -> dict | None:
-    """Sets the tuned tail configuration of `mesh` (a voluma_b200.Mesh) from its device's table."""
+    """Sets the tuned tail configuration of `mesh` (a voluma_b200.Mesh) from its device's table, where it
+    differs from the built-in choice."""
     entries = load_table(mesh.ctx.device_name())
     e = lookup(entries, int(mesh.n_cells), int(getattr(mesh, "n_systems", 1)))
     if e is None:
         return None
-    if (e["cluster"], e["max_rows"], e["full_rows"]) != mesh.tail_config():  # setting it re-plans the launches
+    if not e.get("default", False):
         mesh.set_tail(e["cluster"], e["max_rows"], e["full_rows"])
     return e
 
@@ -77,7 +81,7 @@ def apply(mesh) -> dict | None:
 def candidates(level_rows: list, clusters=(1, 2, 4, 8), max_per_thread: int = 4):
     """Configurations that split one system's levels differently: for each cluster size, the tail
     starting at level 0 (whole V-cycle) or at each coarse level whose rows the cluster covers with at
-    most `max_per_thread` rows per thread."""
+    most 1024 * `max_per_thread` rows a CTA."""
     out = []
     n0 = level_rows[0]
     padded = [(n + 31) // 32 * 32 for n in level_rows]  # coarse levels: rows padded to whole warps
@@ -119,10 +123,11 @@ def time_solves(mesh, d, up, b, ctrl, reps: int):
 
 
 def tune_system(mesh, d, up, b, ctrl, reps: int = 5, log=print) -> dict:
-    """Times every distinct tail configuration of a single-system mesh; keeps the fastest on the mesh
-    and returns its table entry."""
+    """Times every distinct tail configuration of a single-system mesh whose tail was never set; keeps the
+    fastest on the mesh and returns its table entry."""
     sizes = [int(L["n"]) for L in mesh.gamg_levels()]
-    default = mesh.tail_config()
+    cl = mesh.tail_config()[0]
+    default = (cl, 1024 * cl, 2048 if cl == 1 else 1024 * cl)  # the built-in limits, spelled out
     base, x0, it0 = time_solves(mesh, d, up, b, ctrl, reps)
     best = (base, default)
     log(f"  default {default}: {base:.3f} ms, {it0} iterations")
@@ -132,12 +137,12 @@ def tune_system(mesh, d, up, b, ctrl, reps: int = 5, log=print) -> dict:
         # a launch configuration must not change a result: anything else is a defect, never a candidate
         same = it == it0 and np.array_equal(x, x0)
         log(f"  {cfg}: {t:.3f} ms{'' if same else '  RESULT DIFFERS - rejected'}")
-        if same and t < best[0]:
+        if same and t < min(best[0], (1.0 - MARGIN) * base):
             best = (t, cfg)
         if not same:
             raise RuntimeError(f"tail configuration {cfg} changed the solution ({it} vs {it0} iterations)")
     mesh.set_tail(*best[1])
-    return {"rows0": sizes[0], "nsys": 1, "cluster": int(best[1][0]), "max_rows": int(best[1][1]),
+    return {"rows0": sizes[0], "nsys": 1, "default": best[1] == default, "cluster": int(best[1][0]), "max_rows": int(best[1][1]),
             "full_rows": int(best[1][2]), "ms": best[0], "default_ms": base, "levels": sizes}
 
 
