@@ -261,9 +261,8 @@ vlm_status vlm_mesh_stats(vlm_mesh* mesh, int64_t* launches, int64_t* device_byt
  * thread-block cluster of `cluster` CTAs (1, 2, 4 or 8), in its shared memory where the levels fit.
  * 0 keeps a value; row limits left at 0 scale with the cluster.  A mesh whose cluster was never set takes
  * one as wide as the number of systems allows, one CTA for the smallest systems; vlm_mesh_get_tail
- * reports the width in use.  Set it before the mesh's first solve or flow (recorded graphs are dropped; a
- * flow created before keeps launching the old configuration).  The tuner (voluma_b200/tune.py) picks
- * these per device and mesh size. */
+ * reports the width in use.  Recorded graphs of the mesh, its pressure loops and its flows are recorded
+ * again at their next call.  The tuner (voluma_b200/tune.py) picks these per device and mesh size. */
 vlm_status vlm_mesh_set_tail(vlm_mesh* mesh, int32_t cluster, int64_t max_rows, int64_t full_rows);
 vlm_status vlm_mesh_get_tail(vlm_mesh* mesh, int32_t* cluster, int64_t* max_rows, int64_t* full_rows);
 /* Fused launches on the V-cycle's Jacobi levels (no reference counterpart; results bit for bit as

@@ -100,3 +100,25 @@ def test_pressure_corrector_graph_replays_the_direct_run(systems, precision):
     for p, flux, rec in runs[1:]:
         assert np.array_equal(p, runs[0][0]) and np.array_equal(flux, runs[0][1])
         assert rec == runs[0][2]
+
+
+def test_pressure_corrector_graph_after_a_new_tail(systems):
+    """Tail and fusion settings replace what the recorded corrector holds: it is recorded again, with the
+    same results."""
+    ctrl = vb.SolverControls("PCG", "GAMG", 0.0, 1e-8, 500)
+    meshes = [m for m, _ in systems]
+    B = vb.Mesh.batch(meshes)
+    gamma = cases.batch_face_array(meshes, [np.ones(m["n_faces"]) for m in meshes])
+    div = np.concatenate([d for _, d in systems])
+    out = []
+    for k in range(9):
+        if k == 3:
+            B.set_tail(1, 32, 1)
+        if k == 6:
+            B.set_tail(8, 2048, 4096)
+            B.set_fusion(64, 64, 64)
+        p = np.zeros(B.n_cells)
+        _, flux = vb.pressure_solve(B, gamma, div, p, ctrl, ref_cell=[0] * len(meshes), n_non_orth=2, grad_scheme=1)
+        out.append((p, flux))
+    for p, flux in out[1:]:
+        assert np.array_equal(p, out[0][0]) and np.array_equal(flux, out[0][1])

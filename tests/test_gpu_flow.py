@@ -167,3 +167,22 @@ def test_cavity64_reproducible_to_convergence_bitwise(cav64):
     assert its == int(cav64["cav64_repro_iters"])
     assert np.array_equal(U, cav64["cav64_repro_U"]) and np.array_equal(p, cav64["cav64_repro_p"])
     assert fnv1a(U) == fnv1a(cav64["cav64_repro_U"]) and fnv1a(p) == fnv1a(cav64["cav64_repro_p"])
+
+
+def test_launch_settings_changed_between_steps():
+    """A new tail or fusion setting replaces buffers that recorded steps hold: they are recorded again, and
+    the fields stay those of an undisturbed flow bit for bit."""
+    m, case = cases.lid_cavity(32, 100.0)
+    U, p, phi, _ = run(m, case, 9)
+    mesh, fl = flow_for(m, case)
+    fl.set_state(None, None)
+    for k in range(9):
+        if k == 3:
+            mesh.set_tail(1, 64, 1)
+        if k == 6:
+            mesh.set_tail(4, 1024, 4096)
+            mesh.set_fusion(64, 64, 64)
+        fl.step(1.0)
+    U2, p2, phi2 = fl.state()
+    fl.close()
+    assert np.array_equal(U, U2) and np.array_equal(p, p2) and np.array_equal(phi, phi2)

@@ -478,6 +478,7 @@ vlm_status vlm_mesh_set_tail(vlm_mesh* m, int32_t cluster, int64_t max_rows, int
     return guarded(m->ctx, [&] {
         setDevice(m->ctx);
         m->batch->setTail(cluster, max_rows, full_rows);
+        m->pgraphs.clear();
     });
 }
 
@@ -508,6 +509,7 @@ vlm_status vlm_mesh_set_fusion(vlm_mesh* m, int64_t pre_rows, int64_t restrict_r
     return guarded(m->ctx, [&] {
         setDevice(m->ctx);
         m->batch->setFusion(pre_rows, restrict_rows, post_rows);
+        m->pgraphs.clear();
     });
 }
 

@@ -1748,6 +1748,11 @@ vlm_step_info DeviceFlow::step(double dt) {
     // The first step runs directly (it creates every lazily built resource); later steps replay one
     // captured graph per (steady, dt, old-time-level) configuration: one launch per step.
     StepGraph* sg = nullptr;
+    if (batchGeneration_ != batch_.launchGeneration()) {  // the mesh's settings changed: start over
+        stepGraphs_.clear();
+        stepsRun_ = 0;
+        batchGeneration_ = batch_.launchGeneration();
+    }
     if (graphOn_ && stepsRun_ >= 1 && batch_.embeddable() && (!uBatch_ || uBatch_->embeddable()))
         sg = stepGraph(copyOld, copyOldOld);
     int64_t stepOwn = 0;

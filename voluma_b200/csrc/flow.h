@@ -111,7 +111,8 @@ private:
     StepGraph* stepGraph(bool copyOld, bool copyOldOld);
     std::vector<std::unique_ptr<StepGraph>> stepGraphs_;
     bool graphOn_ = true;
-    int64_t stepsRun_ = 0;
+    int64_t stepsRun_ = 0;          // since the step graphs were last dropped
+    int64_t batchGeneration_ = 0;   // the batch's launches that the step graphs hold
     void* pinned_ = nullptr;  // per-step read-back: continuity error, solver records, status words
 
     DeviceBatch& batch_;

@@ -383,6 +383,7 @@ void DeviceBatch::setFusion(int64_t pre, int64_t restrict, int64_t post) {
     if (restrict >= 0) fuseRestrict_ = restrict;
     if (post >= 0) fusePost_ = post;
     graphs_.clear();
+    ++launchGeneration_;
 }
 
 // Re-plans the coarse tail (cluster size, level row limit, whole-V-cycle row limit; 0 keeps the
@@ -393,6 +394,7 @@ void DeviceBatch::setTail(int cluster, int64_t maxRows, int64_t fullRows) {
     if (fullRows != 0) tailFullRows_ = fullRows;
     VLM_CUDA(cudaStreamSynchronize(stream_));
     graphs_.clear();
+    ++launchGeneration_;
     tailOn_ = false;
     planTail();
     buildChunkLists();

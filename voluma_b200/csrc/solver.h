@@ -148,6 +148,9 @@ public:
     // Coarse-tail configuration (tuning): cluster size 1/2/4/8, level row limit, whole-V-cycle row
     // limit (0 keeps a value); re-plans the batch's launches, same results.
     void setTail(int cluster, int64_t maxRows, int64_t fullRows);
+    // Counts the settings that replaced buffers or launches: graphs of others (a flow's steps) that hold
+    // this batch's launches are recorded again when it has changed.
+    int64_t launchGeneration() const { return launchGeneration_; }
     void setFusion(int64_t pre, int64_t restrict, int64_t post);
     // The next solve() reads b and x only after `ev` (their upload on another stream), so the
     // upload overlaps the matrix set-up.
@@ -289,6 +292,7 @@ private:
     DBuf<float> tailVal32_;
     bool planTailSmem(const std::vector<TailSys>& ts, int cluster);
     int tailClusterFor(int systems);
+    int64_t launchGeneration_ = 0;
     int tailCl_ = 0;                     // CTAs of the tail's cluster asked for (setTail); 0: planTail picks
     int64_t tailMaxRows_ = 0;            // levels of at most this many rows go to the tail (0: scaled default)
     int64_t tailFullRows_ = 0;           // systems of at most this many level-0 rows: whole V-cycle there
