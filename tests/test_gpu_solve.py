@@ -301,6 +301,38 @@ def test_coarse_factor_sizes(shape):
     assert rel(w, ro.gamg_apply(M, d, up, None, r, smoother="mcgs-jacobi", coarse=1)) <= 1e-13
 
 
+def unmerged(shape):
+    """A box whose matching stagnates at once (face weights below every partner threshold): one level."""
+    M = vm.box_mesh(shape)
+    M["magSf"] = -1e6 * M["magSf"]
+    d, up = vm.poisson_matrix(vm.box_mesh(shape))
+    return M, 1.05 * d - 0.1 * np.arange(1, M["n_cells"] + 1) / M["n_cells"], up
+
+
+@pytest.mark.parametrize("shape", [(13, 5, 1), (79, 1, 1), (10, 8, 1), (9, 9, 1), (15, 10, 1)])
+def test_coarse_factor_beyond_64_rows(shape):
+    """Coarsest matrices where matching stagnates above 64 rows: the register factor's last rows and second
+    pass over the columns (65 to 80 rows), and the element-wise factor (81 and 150)."""
+    M, d, up = unmerged(shape)
+    assert [L["n"] for L in ro.hierarchy(M)] == [M["n_cells"]]
+    r = np.random.default_rng(6).standard_normal(M["n_cells"])
+    w = vb.gamg_apply(vb.Mesh.from_arrays(M), d, up, None, r)
+    assert rel(w, ro.gamg_apply(M, d, up, None, r, smoother="mcgs-jacobi", coarse=1)) <= 1e-13
+
+
+def test_coarse_factor_of_a_batch_with_one_large_system():
+    """One coarsest matrix beyond the register factor's rows sends the batch's level to the element-wise one."""
+    ms = [unmerged(s) for s in ((15, 10, 1), (8, 8, 1), (3, 3, 1))]
+    r = [np.random.default_rng(7 + i).standard_normal(q[0]["n_cells"]) for i, q in enumerate(ms)]
+    B = vb.Mesh.batch([q[0] for q in ms])
+    w = vb.gamg_apply(B, np.concatenate([q[1] for q in ms]), np.concatenate([q[2] for q in ms]), None, np.concatenate(r))
+    off = 0
+    for (M, d, up), ri in zip(ms, r):
+        wo = ro.gamg_apply(M, d, up, None, ri, smoother="mcgs-jacobi", coarse=1)
+        assert rel(w[off:off + M["n_cells"]], wo) <= 1e-13
+        off += M["n_cells"]
+
+
 def test_64cubed_gamg_against_oracle():
     M = vm.box_mesh((64, 64, 64), hi=(2 * np.pi,) * 3, periodic=(1, 1, 1))
     d, up = vm.poisson_matrix(M)
@@ -480,10 +512,11 @@ def test_cluster_tail_default_start_matches_global_tail(shape, periodic, smoothe
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("systems", [3, 20, 40, 80])
-def test_tail_cluster_widths_of_a_batch_match_solo(systems):
+@pytest.mark.parametrize("systems,width", [(3, 8), (20, 4), (40, 2), (80, 1)])
+def test_tail_cluster_widths_of_a_batch_match_solo(systems, width):
     """More systems take narrower clusters (8, 4, 2 CTAs, one): each system's solution is its own."""
-    shapes = [(6 + q % 5, 7 + q % 3, 5 + q % 4) for q in range(systems)]
+    n = 10 if systems == 3 else 6  # beyond 512 rows somewhere: smaller batches would take one CTA a system
+    shapes = [(n + q % 5, 7 + q % 3, n - 1 + q % 4) for q in range(systems)]
     meshes = [vm.box_mesh(s) for s in shapes]
     rng = np.random.default_rng(8)
     data = []
@@ -492,6 +525,7 @@ def test_tail_cluster_widths_of_a_batch_match_solo(systems):
         b = rng.standard_normal(M["n_cells"])
         data.append((d, up, b - b.mean()))
     B = vb.Mesh.batch(meshes)
+    assert B.tail_config()[0] == width
     c = ctrl(preconditioner="GAMG")
     x = np.zeros(B.n_cells)
     vb.solve_ldu(B, *(np.concatenate([q[k] for q in data]) for k in (0, 1)), None,
