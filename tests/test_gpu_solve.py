@@ -394,7 +394,7 @@ def test_tail_launch_configurations_give_identical_results(name, precision):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("shape,auto", [((20, 20, 20), 8), ((9, 7, 5), 1)])
+@pytest.mark.parametrize("shape,auto", [((20, 20, 20), 8), ((12, 10, 9), 8), ((9, 7, 5), 1), ((32, 32, 1), 1)])
 def test_tail_width_can_be_asked_for(shape, auto, monkeypatch):
     """The planner's width is reported, every width can be asked for, in shared and in global memory, and
     none changes the solution; 0 keeps the width that was asked for."""
@@ -515,7 +515,7 @@ def test_cluster_tail_default_start_matches_global_tail(shape, periodic, smoothe
 @pytest.mark.parametrize("systems,width", [(3, 8), (20, 4), (40, 2), (80, 1)])
 def test_tail_cluster_widths_of_a_batch_match_solo(systems, width):
     """More systems take narrower clusters (8, 4, 2 CTAs, one): each system's solution is its own."""
-    n = 10 if systems == 3 else 6  # beyond 512 rows somewhere: smaller batches would take one CTA a system
+    n = 6 if systems == 80 else 14  # beyond 1,024 rows somewhere: smaller batches take one CTA a system
     shapes = [(n + q % 5, 7 + q % 3, n - 1 + q % 4) for q in range(systems)]
     meshes = [vm.box_mesh(s) for s in shapes]
     rng = np.random.default_rng(8)

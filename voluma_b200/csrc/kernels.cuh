@@ -975,8 +975,8 @@ __global__ void k_coarse_apply(const CoarseDev* __restrict__ cs, const double* _
 // the result is bit-identical to the per-level launch sequence.
 constexpr int kTailThreads = 1024;
 constexpr int kTailBatch = 4;      // entries in flight per row (64 registers at 1024 threads)
-constexpr int kTailMaxRows = 1024;  // levels at most this many rows (padded) go to the tail
-constexpr int kTailFullRows = 2048;  // systems at most this many level-0 rows run the whole V-cycle there
+constexpr int kTailMaxRows = 1024;  // levels of at most this many rows (padded) per CTA go to the tail
+constexpr int kTailFullRows = 2048;  // one CTA: systems of at most this many level-0 rows run whole V-cycles there
 
 // CL: CTAs of the thread-block cluster that runs one system's tail (CL == 1: one CTA).  With CL > 1
 // the rows of each step are spread over the cluster's threads and the steps are separated by the

@@ -1095,7 +1095,10 @@ int tailClusters() {
 // alone; the whole V-cycle for systems of at most the full-row limit.  The tail runs in shared memory on
 // one cluster per system: of the width asked for, else as wide as lets every system's cluster be
 // resident at once (tailClusterFor); in global memory where the coarsest levels do not fit.  Limits that
-// are not set scale with the width.
+// are not set scale with the width: 1,024 padded rows per CTA (kTailMaxRows, two per thread).  What the
+// limit decides is whether a level of 1,700 to 8,192 rows still runs in the tail; solves at mixed precision
+// with it and without, ms: 96^3 (3,413 rows) 8.12 / 8.72, 64^3 (4,032) 3.70 / 3.96, 48^3 (6,848) 3.48 /
+// 3.63, 256^2 (4,064) 5.25 / 5.64, and the whole of 64^2 1.55 / 1.64.  Larger levels do not fit.
 void DeviceBatch::planTail() {
     const char* tv = std::getenv("VLM_TAIL");
     if (tv && tv[0] == '0') return;
@@ -1162,10 +1165,17 @@ void DeviceBatch::planTail() {
     } else if (tailSmemAllowed_) {
         int cluster = tailClusterFor(ns);
         std::vector<TailSys> ts = starts(cluster);
-        // at most one row per thread of one CTA on every level: its own barrier is shorter than the
-        // cluster's (480 cells, 11 iterations: 0.65 -> 0.61 ms a solve).  Running only the levels below
-        // 512 rows of a larger tail that way measured slower (96^3 FP64 11.26 -> 11.39 ms).
-        if (std::all_of(ts.begin(), ts.end(), [](const TailSys& t) { return t.rowCount[t.first] <= kTailPartThreads; })) {
+        // At most two rows per thread of one CTA on every level, and images that fit it: its own barrier is
+        // shorter than the cluster's.  FP64 solves, ms (medians over ten registrations: where the buffers
+        // land moves such a solve by 4%), 8 CTAs against one: 560 cells 0.626 / 0.572, 800 0.750 / 0.727,
+        // 32 x 32 0.769 / 0.703, 1000 0.796 / 0.795, 1152 0.857 / 0.876, 2048 0.927 / 0.984; FP32 one CTA
+        // ahead to 1568.  Running only the levels below 512 rows of a larger tail on one CTA measured
+        // slower (96^3 FP64 11.26 -> 11.39 ms).
+        std::vector<int> first;
+        size_t bytes = 0;
+        if (std::all_of(ts.begin(), ts.end(), [](const TailSys& t) { return t.rowCount[t.first] <= 2 * kTailPartThreads; }) &&
+            tailStarts(plan_, ts, 1, sizeof(double), size_t(tailBudget()), first, bytes) &&
+            std::equal(ts.begin(), ts.end(), first.begin(), [](const TailSys& t, int f) { return t.first == f; })) {
             tailClusters<1>();
             cluster = 1;
         }
