@@ -5,10 +5,11 @@
 // meets no barrier but its own: it streams its steps' rows and entries into a shared-memory ring with
 // cp.async, keeps its swept vector in shared memory, and receives the values of other parts through
 // mailboxes of 16 bytes {value, launch number}, written and read whole, which need neither a fence
-// nor a flag.  A mailbox is polled two steps before its value is used, so a hand-over costs latency
-// once per part (parts run staggered) and not once per level.  Measured: one PBiCGStab/DILU solve of
-// 80 x 64 x 48 cells (a factorisation and six applications, 190 levels each way) 14.6 -> 5.2 ms; the
-// Taylor-Green step at 64^3 15.1 -> 9.4 ms, the 96 x 72 x 48 LES channel step 39.9 -> 19.7 ms.
+// nor a flag.  A mailbox is read two steps before its value is used and polled again when it was empty.
+// Measured: one PBiCGStab/DILU solve of 80 x 64 x 48 cells (a factorisation and six applications, 190
+// levels each way) 13.8 ms with the barrier per level, 5.2 with k_dilu_part and 3.1 with k_dilu_pipe below,
+// which takes such meshes; k_dilu_part alone: a column of 20,000 cells (two parts, one after the other)
+// 0.85 us a level, 150 x 140 x 130 cells (418 levels, its vectors in global memory) 2.3 us a level.
 //
 // Parts only wait for parts of an earlier ticket, and tickets are taken in the order in which CTAs
 // start, so a sweep ends however few of its CTAs are resident; no cooperative launch.  On a mesh that is
@@ -278,9 +279,11 @@ __global__ void __launch_bounds__(kPartThreads, 1) k_dilu_part(const DiluPartArg
 
 // ---------------------------------------------------------------- records
 // The same sweep for rows of at most six neighbours per direction (box meshes) whose parts' vectors fit in
-// shared memory.  What bounds it is one CTA's path through a step: 0.17-0.25 us against 1.7 us of
-// k_dilu_part, whose entry loop (a dependent load of the column, a choice of source and a load of the
-// value per entry) and step descriptors read from global memory took 3,000 cycles a step.  Here a row is
+// shared memory.  What bounds it is the latency of a level: 0.9-1.3 us in a solve (33 x 39 x 35 0.86, 80 x
+// 64 x 48 1.03, 64^3 1.15, 96 x 72 x 48 1.27), with one issue slot in ten used and 44% of the warps' time at
+// the step's barrier (ncu at 33 x 39 x 35: 1.2 us a level with cold caches, where the one-CTA kernels of
+// dilu.cuh, which wait for nobody, take 0.47 at 64^2).  In k_dilu_part each entry is a dependent load of
+// the column, a choice of source and a load of the value.  Here a row is
 // one 16-byte word of columns, one 32-byte word of coefficients with 1 / rD, and three values at
 // once; a few rows (periodic links) read a second record.  Everything a step needs from global
 // memory is requested at least two steps before.

@@ -1449,7 +1449,9 @@ void DeviceBatch::recordBicgIterT(PrecondKind pk, SmootherKind sm, bool f32) {
 // ====================================================================== level-scheduled paths
 // The pipelined schedule.  A part gets about kPartWidth rows of a full level (one per thread, with
 // room for uneven cuts), and no more rows than its vector's share of shared memory: more parts would
-// lengthen the start-up of the pipeline, fewer would split levels into several steps.  Packed records
+// lengthen the start-up of the pipeline, fewer would split levels into several steps.  A PBiCGStab
+// iteration at 128 / 160 / 192 / 224 / 256 rows, us: 61 x 61 x 41 cells 631 / 622 / 616 / 629 / 629, 33 x 39
+// x 35 400 / 391 / 391 / 392 / 474; larger meshes' parts are as many as their vectors need.  Packed records
 // where every row has at most six entries per direction and the parts' vectors fit with a ring of
 // three stages at least; else the general kernel, with its vectors in global memory where a system
 // would need more parts than SMs.
