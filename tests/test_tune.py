@@ -39,3 +39,24 @@ def test_committed_table_shape():
         for e in t["entries"]:
             assert e["cluster"] in (1, 2, 4, 8) and e["max_rows"] >= 0 and e["full_rows"] >= 0
             assert e["ms"] <= e["default_ms"] * 1.001  # the kept configuration is never slower than the default
+
+
+def test_apply_leaves_the_planner_alone_where_it_is_the_fastest(monkeypatch):
+    class Ctx:
+        def device_name(self):
+            return "some device"
+
+    class Mesh:
+        ctx, n_cells, n_systems = Ctx(), 4096, 1
+        calls = []
+
+        def set_tail(self, *cfg):
+            self.calls.append(cfg)
+
+    kept = dict(rows0=4096, nsys=1, default=True, cluster=8, max_rows=8192, full_rows=8192)
+    tuned = dict(kept, default=False, cluster=2, max_rows=256)
+    m = Mesh()
+    monkeypatch.setattr(tune, "load_table", lambda name: [kept])
+    assert tune.apply(m) is kept and m.calls == []
+    monkeypatch.setattr(tune, "load_table", lambda name: [tuned])
+    assert tune.apply(m) is tuned and m.calls == [(2, 256, 8192)]

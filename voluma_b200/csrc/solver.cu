@@ -1478,6 +1478,8 @@ void DeviceBatch::planDiluParts(DiluDev& D, const DiluPlan& P, int sms) {
     constexpr size_t kSmemMax = 220 * 1024;
     DiluParts R;
     DiluRecords C;
+    D.records = D.local = false;  // (an earlier attempt may have run out of memory)
+    D.nLoS = D.nUpS = 0;
     // the parts for at most maxSlots slots each (0: any) and steps of at most W rows; one: a part per system
     auto plan = [&](int maxSlots, int W, bool one) {
         std::vector<int> np(P.sys.size(), 1);
